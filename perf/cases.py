@@ -32,32 +32,32 @@ HIT_COLUMNS = ("pos", "time", "dir0", "weight", "dir", "wavelength", "dist", "pa
 def listed():
     return [
         # the isotropic point source that also runs on a CPU: one small call, all latency
-        {"name": "point source, 1e5 photons", "kind": "propagate_host", "pairs": 1, "n_min": 1e5, "n_max": 1e5,
+        {"name": "point-1e5", "kind": "propagate_host", "pairs": 1, "n_min": 1e5, "n_max": 1e5,
          "d_min": 10.0, "d_max": 10.0, "cone": 0.0, "bins": 500, "mode": "physical"},
         # one request of the serving stream: tens of uneven pairs, isotropic and cone emitters
-        {"name": "request, 33 pairs", "kind": "propagate_host", "pairs": 33, "n_min": 1e4, "n_max": 1e6,
+        {"name": "request-33-pairs", "kind": "propagate_host", "pairs": 33, "n_min": 1e4, "n_max": 1e6,
          "d_min": 2.0, "d_max": 150.0, "cone": 0.5, "bins": 1000, "mode": "physical"},
         # the headline batch
-        {"name": "mixed batch, 4096 pairs", "kind": "propagate_device", "pairs": 4096, "n_min": 1e4, "n_max": 1e7,
+        {"name": "mixed-4096-pairs", "kind": "propagate_device", "pairs": 4096, "n_min": 1e4, "n_max": 1e7,
          "d_min": 2.0, "d_max": 150.0, "cone": 0.5, "bins": 1000, "gev": 0.0},
         # a 10 GeV shower: 200 cascade-profile sources x 500 modules, about 1e4 photons per pair
-        {"name": "event, 1e5 cascade pairs", "kind": "propagate_device", "pairs": 0, "n_min": 0.0, "n_max": 0.0,
+        {"name": "event-1e5-cascade-pairs", "kind": "propagate_device", "pairs": 0, "n_min": 0.0, "n_max": 0.0,
          "d_min": 0.0, "d_max": 0.0, "cone": 0.0, "bins": 1000, "gev": 10.0},
         # a quick fit table, and a large one whose hits take a share of the time
-        {"name": "fits, 20 distances x 25 angles", "kind": "fits", "photons": 1000000, "distances": 20, "angles": 25},
-        {"name": "fits, 100 distances x 250", "kind": "fits", "photons": 20000000, "distances": 100, "angles": 250},
+        {"name": "fits-20x25", "kind": "fits", "photons": 1000000, "distances": 20, "angles": 25},
+        {"name": "fits-100x250", "kind": "fits", "photons": 20000000, "distances": 100, "angles": 250},
         # surrogate queries: a full batch, and the few thousand of a small detector (ragged)
-        {"name": "queries, 1e6", "kind": "forward", "n": 1000000},
-        {"name": "queries, 3001", "kind": "forward", "n": 3001},
+        {"name": "queries-1e6", "kind": "forward", "n": 1000000},
+        {"name": "queries-3001", "kind": "forward", "n": 3001},
         # one Adam step at the batch the surrogate is trained with
-        {"name": "training step, 4096 rows", "kind": "train", "n": 4096},
+        {"name": "train-4096", "kind": "train", "n": 4096},
         # training targets of one chunk of pairs
-        {"name": "mixture fit, 20000 pairs", "kind": "mixture", "n": 20000, "bins": 1000, "iters": 60},
+        {"name": "mixture-20000", "kind": "mixture", "n": 20000, "bins": 1000, "iters": 60},
         # 64 energy hypotheses of a 100 GeV shower
-        {"name": "likelihood, 64 hypotheses", "kind": "llh", "hypotheses": 64, "modules": 500, "sources": 200,
+        {"name": "likelihood-64", "kind": "llh", "hypotheses": 64, "modules": 500, "sources": 200,
          "hits": 46000, "mode": "shifted"},
         # the same shower's sources, and a pair with every module
-        {"name": "sources and pairs, 1 particle", "kind": "lightyield", "particles": 1, "intervals": 200,
+        {"name": "sources-and-pairs", "kind": "lightyield", "particles": 1, "intervals": 200,
          "modules": 500},
     ]
 
