@@ -183,7 +183,8 @@ struct DevTables {
   int32_t n_knots;
   int32_t n_abs;
   int32_t n_pmt;
-  int32_t pad0, pad1;
+  int32_t n_cells;  // intervals of the knots: n_knots - 1, or 1 with knots[1] = knots[0] for a single wavelength
+  int32_t pad0;
   float knots[PP_MAX_KNOTS];
   float abs_wl[PP_MAX_ABS];
   float abs_len[PP_MAX_ABS];
@@ -229,12 +230,12 @@ __device__ __forceinline__ float interp_sorted(float x, const float* xs, const f
   return fmaf(ys[hi] - ys[lo], along, ys[lo]);
 }
 
-// fast_linear_interp(u, knots, 0, 1) for u in (0, 1) (src/utils.jl:37-60).
+// fast_linear_interp(u, knots, 0, 1) for u in (0, 1) (src/utils.jl:37-60); a
+// single wavelength is one interval of width 0, which gives it exactly.
 __device__ __forceinline__ float draw_wavelength(const DevTables& T, float u) {
-  if (T.n_knots == 1) return T.knots[0];
-  const float x = u * (float)(T.n_knots - 1);
+  const float x = u * (float)T.n_cells;
   int i = (int)x;
-  i = min(i, T.n_knots - 2);
+  i = min(i, T.n_cells - 1);
   const float f = x - (float)i;
   return fmaf(T.knots[i + 1] - T.knots[i], f, T.knots[i]);
 }
@@ -264,14 +265,26 @@ __device__ __forceinline__ float cascade_cos_theta(const DevTables& T, float c0,
 // are left out of the step.
 struct HG {
   float two_g, one_m_g, a, one_p_g2, inv_2g;
-  int iso;
+  float iso_a, iso_b;
 };
-// g == 0 (isotropic, where the formula divides by zero) is a select rather
-// than a branch: the formula then gives 0 (inv_2g is 0), which is dropped.
+// g == 0 (isotropic, where the formula divides by zero) needs no branch or
+// select: the formula's term is then 0 (inv_2g is 0) and iso_a u + iso_b is
+// 2 u - 1; for any other g iso_a = iso_b = 0 add nothing.
+__host__ __device__ __forceinline__ HG make_hg(float g) {
+  HG h;
+  const bool iso = g == 0.f;
+  h.two_g = 2.f * g;
+  h.one_m_g = 1.f - g;
+  h.a = 1.f - g * g;
+  h.one_p_g2 = 1.f + g * g;
+  h.inv_2g = iso ? 0.f : 1.f / (2.f * g);
+  h.iso_a = iso ? 2.f : 0.f;
+  h.iso_b = iso ? -1.f : 0.f;
+  return h;
+}
 __device__ __forceinline__ float hg_costheta(const HG& h, float u) {
   const float t = h.a * rcp(fmaf(h.two_g, u, h.one_m_g));
-  const float c = fmaf(-t, t, h.one_p_g2) * h.inv_2g;
-  return h.iso ? fmaf(2.f, u, -1.f) : c;
+  return fmaf(h.iso_a, u, fmaf(fmaf(-t, t, h.one_p_g2), h.inv_2g, h.iso_b));
 }
 
 // Rotation that takes e_z to the unit vector o, applied to n (the Rodrigues
@@ -358,6 +371,7 @@ struct Photon {
   uint32_t sc0;       // the step stream (from the emission block): counter word 0
   uint32_t sc1;       // and the base added to ctr3 for counter word 1
   uint32_t id_lo;     // photon index bits 0..31 (bits 32..39 are the low byte of ctr3)
+  float a, q;         // line_of: the next step's ray-sphere test (physical mode: made when the photon stopped)
 };
 
 // The photon's index: bits 0..31 in id_lo, 32..39 in the low byte of ctr3
@@ -373,91 +387,38 @@ __device__ __forceinline__ void set_photon(Photon& s, uint64_t id) {
 
 struct PairCtx {
   float r;  // sphere radius
-  uint32_t seed_lo, seed_hi;
   int32_t index;
 };
 
-__device__ __forceinline__ PairCtx load_pair_ctx(const pp_pair* __restrict__ P, int index) {
-  const uint2 sd = __ldg(reinterpret_cast<const uint2*>(P) + 7);  // seed
-  PairCtx c;
-  c.r = __ldg(reinterpret_cast<const float*>(P) + 11);  // radius
-  c.seed_lo = sd.x;
-  c.seed_hi = sd.y;
-  c.index = index;
-  return c;
-}
-
-__device__ __forceinline__ float3 pair_target(const pp_pair* __restrict__ P) {
-  const float4 t = __ldg(reinterpret_cast<const float4*>(P) + 2);  // target, radius
-  return make_float3(t.x, t.y, t.z);
-}
-
-// Where and how a photon is emitted, from block 0 of its stream
-// (src/photon_prop_cuda.jl:52-56, 67-75, 308-316).  The emission direction
-// is written as a polar angle about an axis, like a scattering: isotropic
-// emission is polar angle acos(2 u1 - 1) about e_z; the Cherenkov cone (no
-// reference code) is acos(1/n(wl)) about the track, from a point uniform
-// along the track at time t0 + s/c.  The reference-compatible isotropic
-// draw takes theta = 2 u1 - 1 radians (a reference quirk) and so carries its
-// own sin(theta).
-struct EmissionFrame {
-  float px, py, pz, t_emit, wl;
-  float ox, oy, oz;  // polar axis
-  float cpol, spol;  // spol valid only if has_spol
-  bool has_spol;
-  bool axis_ez;  // isotropic: the axis is e_z
+// What an emission reads of a pair record.
+struct PairRec {
+  float4 pos_t0, dir_len, tgt_r;
+  uint32_t seed_lo, seed_hi;
+  int32_t emitter;
 };
 
-// EM selects the emitters a kernel variant samples: 0 isotropic and cone
-// (a cascade pair is then emitted on the cone; the batched kernel flags it),
-// kEmCascade also the cascade profile, whose table lookups would otherwise
-// cost every variant registers.
-enum { kEmBasic = 0, kEmCascade = 1 };
-
-template <int MODE, int EM = kEmBasic>
-__device__ __forceinline__ EmissionFrame emission_frame(const DevTables& T, const pp_pair* __restrict__ P,
-                                                        const Draw3& d) {
-  const float4 pt = __ldg(reinterpret_cast<const float4*>(P));      // pos, t0
-  const float4 dl = __ldg(reinterpret_cast<const float4*>(P) + 1);  // dir, track_len
-  const int emitter = __ldg(reinterpret_cast<const int*>(P) + 16);
-  EmissionFrame f;
-  f.wl = draw_wavelength(T, d.u0);
-  f.px = pt.x;
-  f.py = pt.y;
-  f.pz = pt.z;
-  f.t_emit = pt.w;
-  f.has_spol = false;
-  f.spol = 0.f;
-  f.axis_ez = emitter == PP_EMITTER_ISOTROPIC;
-  if (emitter == PP_EMITTER_ISOTROPIC) {
-    f.ox = 0.f;
-    f.oy = 0.f;
-    f.oz = 1.f;
-    if (MODE == kCompat) {
-      const float th = fmaf(2.f, d.u1, -1.f);
-      f.cpol = cos_a(th);
-      f.spol = sin_a(th);
-      f.has_spol = true;
-    } else {
-      f.cpol = fmaf(2.f, d.u1, -1.f);
-    }
-  } else {  // Cherenkov cone (a track), or the cascade profile (a point)
-    f.ox = dl.x;
-    f.oy = dl.y;
-    f.oz = dl.z;
-    const float c0 = rcp(phase_index(T, rcp(f.wl)));
-    f.cpol = c0;
-    float s = d.u1 * dl.w;
-    if (EM == kEmCascade && emitter == PP_EMITTER_CASCADE) {
-      f.cpol = cascade_cos_theta(T, c0, d.u1);
-      s = 0.f;
-    }
-    f.px = fmaf(s, f.ox, f.px);
-    f.py = fmaf(s, f.oy, f.py);
-    f.pz = fmaf(s, f.oz, f.pz);
-    f.t_emit = fmaf(s, 1.f / kCVac, f.t_emit);
-  }
-  return f;
+__device__ __forceinline__ PairRec load_pair(const pp_pair* __restrict__ P) {
+  PairRec r;
+  r.pos_t0 = __ldg(reinterpret_cast<const float4*>(P));
+  r.dir_len = __ldg(reinterpret_cast<const float4*>(P) + 1);
+  r.tgt_r = __ldg(reinterpret_cast<const float4*>(P) + 2);
+  const uint2 sd = __ldg(reinterpret_cast<const uint2*>(P) + 7);
+  r.seed_lo = sd.x;
+  r.seed_hi = sd.y;
+  r.emitter = __ldg(reinterpret_cast<const int*>(P) + 16);
+  return r;
+}
+// the same from a copy of the record in shared memory
+__device__ __forceinline__ PairRec staged_pair(const float4* rec) {
+  PairRec r;
+  r.pos_t0 = rec[0];
+  r.dir_len = rec[1];
+  r.tgt_r = rec[2];
+  const uint2 sd = reinterpret_cast<const uint2*>(rec)[7];
+  r.seed_lo = sd.x;
+  r.seed_hi = sd.y;
+  r.emitter = reinterpret_cast<const int*>(rec)[16];
+  return r;
 }
 
 // Unit vector at polar cos cpol (sin spol) and azimuth 2 pi u about the axis o
@@ -505,19 +466,58 @@ __device__ __forceinline__ void scatter_turn(float ux, float uy, float uz, float
   rz = fmaf(-a, s2 * rs, uz * cpol);
 }
 
-// Emission direction of a frame: the isotropic axis is e_z, about which the
-// polar vector needs no rotation; the cone axis is the track.
-__device__ __forceinline__ void emission_direction(const EmissionFrame& f, float u, float& rx, float& ry,
-                                                   float& rz) {
-  const float spol = f.has_spol ? f.spol : sin_from_cos(f.cpol);
-  if (f.axis_ez) {
-    const float ph = fmaf(kTwoPi, u, -kPi);
-    rx = -cos_a(ph) * spol;
-    ry = -sin_a(ph) * spol;
-    rz = f.cpol;
-  } else {
-    polar_direction(f.ox, f.oy, f.oz, f.cpol, spol, u, rx, ry, rz);
+// Where and how a photon is emitted, from block 0 of its stream
+// (src/photon_prop_cuda.jl:52-56, 67-75, 308-316).  The emission direction
+// is a polar angle and an azimuth about an axis, like a scattering: isotropic
+// emission is polar angle acos(2 u1 - 1) about e_z (no rotation); the
+// Cherenkov cone (no reference code) is acos(1/n(wl)) about the track, from a
+// point uniform along the track at time t0 + s/c.  The reference-compatible
+// isotropic draw takes theta = 2 u1 - 1 radians (a reference quirk) and so
+// carries its own sin(theta).
+struct EmissionFrame {
+  float px, py, pz, t_emit, wl;
+  float rx, ry, rz;  // emission direction
+};
+
+// EM selects the emitters a kernel variant samples: 0 isotropic and cone
+// (a cascade pair is then emitted on the cone; the batched kernel flags it),
+// kEmCascade also the cascade profile, whose table lookups would otherwise
+// cost every variant registers.
+enum { kEmBasic = 0, kEmCascade = 1 };
+
+template <int MODE, int EM = kEmBasic>
+__device__ __forceinline__ EmissionFrame emission_frame(const DevTables& T, const PairRec& P, const Draw3& d) {
+  const float4 pt = P.pos_t0;
+  const float4 dl = P.dir_len;
+  EmissionFrame f;
+  f.wl = draw_wavelength(T, d.u0);
+  if (P.emitter == PP_EMITTER_ISOTROPIC) {
+    f.px = pt.x;
+    f.py = pt.y;
+    f.pz = pt.z;
+    f.t_emit = pt.w;
+    const float th = fmaf(2.f, d.u1, -1.f);
+    const float cpol = MODE == kCompat ? cos_a(th) : th;
+    const float spol = MODE == kCompat ? sin_a(th) : sin_from_cos(cpol);
+    const float ph = fmaf(kTwoPi, d.u2, -kPi);
+    f.rx = -cos_a(ph) * spol;
+    f.ry = -sin_a(ph) * spol;
+    f.rz = cpol;
+  } else {  // Cherenkov cone (a track), or the cascade profile (a point)
+    const float c0 = rcp(phase_index(T, rcp(f.wl)));
+    float cpol = c0;
+    float s = d.u1 * dl.w;
+    if (EM == kEmCascade && P.emitter == PP_EMITTER_CASCADE) {
+      cpol = cascade_cos_theta(T, c0, d.u1);
+      s = 0.f;
+    }
+    f.px = fmaf(s, dl.x, pt.x);
+    f.py = fmaf(s, dl.y, pt.y);
+    f.pz = fmaf(s, dl.z, pt.z);
+    f.t_emit = fmaf(s, 1.f / kCVac, pt.w);
+    polar_direction(dl.x, dl.y, dl.z, cpol, sin_from_cos(cpol), d.u2, f.rx, f.ry, f.rz);
   }
+  return f;
 }
 
 // Path a photon emitted in frame f can travel before t_max at the group
@@ -527,100 +527,128 @@ __device__ __forceinline__ float path_at_tmax(const DevTables& T, const RunParam
   return (R.t_max - f.t_emit) * kCVac * rcp(group_index(T, rcp(f.wl)));
 }
 
+// The line from the photon along its direction against the sphere: a, the
+// (negative) path to the point nearest the centre, and q, that point's squared
+// distance from it.  The ray-sphere discriminant
+// a^2 - |e|^2 + r^2 (src/photon_prop_cuda.jl:340) is r^2 - q = r^2 - |e - a d|^2:
+// the same number, but without cancelling two large squares, which in FP32
+// costs millimetres at grazing incidence on a sphere tens of metres away.
+// (x, y) pairs on sm_100's packed FP32 instructions (round to nearest: the
+// scalar results bit for bit, in half the issue slots).
+__device__ __forceinline__ void line_of(Photon& s) {
+  s.a = fmaf(s.dz, s.pz, fmaf(s.dy, s.py, s.dx * s.px));
+  const float2 qxy = __ffma2_rn(make_float2(-s.a, -s.a), make_float2(s.dx, s.dy), make_float2(s.px, s.py));
+  const float qz = fmaf(-s.a, s.dz, s.pz);
+  s.q = fmaf(qz, qz, fmaf(qxy.y, qxy.y, qxy.x * qxy.x));
+}
+
+// Physical mode: a photon farther from the sphere than the path it has left
+// before t_max can never arrive in time (any path to the sphere is at least
+// the straight distance).  Exact, with a margin for FP32 rounding; it spares
+// the steps of photons drifting away from their target.  The test is made as
+// soon as a photon stops (after its emission and after each step's turn), so
+// that its lane is free for another photon at once: 87 % of the photons of
+// the 4096-pair mixed batch end this way, and tested at the head of the next
+// step each of them took a whole step (a Philox block, a move, a turn) only
+// to find this out: 0.87 of 4.24 steps per photon.
+__device__ __forceinline__ bool in_reach(const Photon& s, float r) {
+  const float pp = fmaf(s.a, s.a, s.q);  // |e|^2
+  const float reach = fmaf(s.path, 1.0001f, r + 0.05f);
+  return pp <= reach * reach;
+}
+
 // Emission of photon photon_index(s) (its emission block): position, direction, the
 // per-wavelength constants and the step stream; afterwards the next event
-// is step 0 (step block 1).
+// is step 0 (step block 1).  Returns false for a photon that is out of reach.
 template <int MODE, int EM = kEmBasic>
-__device__ __forceinline__ void emit_event(const DevTables& T, const RunParams& R, const pp_pair* __restrict__ P,
-                                           const PairCtx& c, Photon& s) {
+__device__ __forceinline__ bool emit_event(const DevTables& T, const RunParams& R, const PairRec& P, Photon& s) {
   const uint64_t id = photon_index(s);
-  const uint4 w = emission_block(c.seed_lo, c.seed_hi, id);
+  const uint4 w = emission_block(P.seed_lo, P.seed_hi, id);
   const Draw3 d = emission_uniforms(w);
   const EmissionFrame f = emission_frame<MODE, EM>(T, P, d);
-  const float3 tg = pair_target(P);
-  s.px = f.px - tg.x;
-  s.py = f.py - tg.y;
-  s.pz = f.pz - tg.z;
+  s.px = f.px - P.tgt_r.x;
+  s.py = f.py - P.tgt_r.y;
+  s.pz = f.pz - P.tgt_r.z;
   s.path = (MODE == kPhysical) ? path_at_tmax(T, R, f) : 0.f;
   s.neg_ln2_len = -kLn2 * scattering_length(T, f.wl);
-  emission_direction(f, d.u2, s.dx, s.dy, s.dz);
+  s.dx = f.rx;
+  s.dy = f.ry;
+  s.dz = f.rz;
   s.sc0 = w.w;
   s.sc1 = step_base(w);
   s.ctr3 = ctr_word(id, 1u);
+  if (MODE == kCompat) return true;
+  line_of(s);
+  return in_reach(s, P.tgt_r.w);
 }
 
 // Step k (block k + 1 of the photon's Philox2x32 stream) of
 // src/photon_prop_cuda.jl:320-376: step length,
 // ray-sphere test, move, Henyey-Greenstein turn.  Returns false when the
 // photon ends; *hit is set when it ends on the sphere (position and path
-// length then at the hit).
+// length then at the hit; a photon that ends otherwise leaves no state that
+// is read).  `more` says whether the photon has another step coming, which
+// for a photon that ends out of reach is the step that would end it: the
+// photon steps of a run are the emissions (each has a first step) plus these.
 template <int MODE>
-__device__ __forceinline__ bool step_event(const RunParams& R, const PairCtx& c, Photon& s, bool& hit) {
+__device__ __forceinline__ bool step_event(const RunParams& R, const PairCtx& c, Photon& s, bool& hit, bool& more) {
   uint32_t w0 = s.sc0, w1 = s.sc1 + s.ctr3;
   philox2x32_10(w0, w1, kStepKey);
   const Draw3 d = step_uniforms(w0, w1);
   const float step = lg2(d.u0) * s.neg_ln2_len;
-  const float ex = s.px, ey = s.py, ez = s.pz;  // photon - sphere centre
-  const float a = fmaf(s.dz, ez, fmaf(s.dy, ey, s.dx * ex));
-  // b = a^2 - |e|^2 + r^2 (src/photon_prop_cuda.jl:340) evaluated as r^2 - |e - a d|^2:
-  // the same number, but without cancelling two large squares, which in FP32
-  // costs millimetres at grazing incidence on a sphere tens of metres away
-  // (x, y) pairs on sm_100's packed FP32 instructions (round to nearest: the
-  // scalar results bit for bit, in half the issue slots)
-  const float2 qxy = __ffma2_rn(make_float2(-a, -a), make_float2(s.dx, s.dy), make_float2(ex, ey));
-  const float qx = qxy.x, qy = qxy.y, qz = fmaf(-a, s.dz, ez);
-  const float q = fmaf(qz, qz, fmaf(qy, qy, qx * qx));
-  const float b = fmaf(c.r, c.r, -q);
-  const float pp = fmaf(a, a, q);  // |e|^2
-  // branch-free decisions: the line meets the sphere (b >= 0) at dd ahead
-  // (b < 0 makes dd NaN, which no decision reads: line is false)
-  const float dd = -a - sqrt_a(b);
-  const bool line = b >= 0.f;
-  const bool geo = line && dd > 0.f && dd < step;  // reaches the sphere within this step
-  bool alive, move;
-  if (MODE == kCompat) {
-    hit = geo;
-    move = !line;  // the line meets the sphere outside this step: no move (reference)
-    alive = !geo;
-  } else {
-    hit = geo && dd <= s.path;  // arrives inside the time window
-    // A photon farther from the sphere than the path it has left before t_max
-    // can never arrive in time (any path to the sphere is at least the straight
-    // distance): it ends now.  Exact, with a margin for FP32 rounding; it
-    // spares the steps of photons drifting away from their target.
-    const float reach = fmaf(s.path, 1.0001f, c.r + 0.05f);
-    move = !geo && step <= s.path && pp <= reach * reach;
-    alive = move;
-  }
-  const float len = hit ? dd : (move ? step : 0.f);
-  const float2 pxy = __ffma2_rn(make_float2(len, len), make_float2(s.dx, s.dy), make_float2(s.px, s.py));
-  s.px = pxy.x;
-  s.py = pxy.y;
-  s.pz = fmaf(len, s.dz, s.pz);
-  s.path += (MODE == kPhysical) ? -len : len;
+  if (MODE == kCompat) line_of(s);  // nothing needs it earlier there, and carried it costs registers
+  const float b = fmaf(c.r, c.r, -s.q);
+  // branch-free decisions: the line meets the sphere (b >= 0) at dd ahead;
+  // b < 0 makes dd NaN, for which every comparison is false
+  const float dd = -s.a - sqrt_a(b);
+  const bool geo = dd > 0.f && dd < step;  // reaches the sphere within this step
   const float cpol = hg_costheta(R.hg, d.u1);
   float rx, ry, rz;
-  if (MODE == kPhysical) {
-    scatter_turn(s.dx, s.dy, s.dz, cpol, sin_from_cos(cpol), d.u2, rx, ry, rz);
-  } else {
-    polar_direction<false>(s.dx, s.dy, s.dz, cpol, sin_from_cos(cpol), d.u2, rx, ry, rz);
-  }
-  s.dx = move ? rx : s.dx;
-  s.dy = move ? ry : s.dy;
-  s.dz = move ? rz : s.dz;
   s.ctr3 += 1u << 8;
-  return alive && s.ctr3 < R.ctr_limit;  // at most max_steps steps
+  if (MODE == kCompat) {
+    hit = geo;
+    const bool move = !(b >= 0.f);  // the line meets the sphere outside this step: no move (reference)
+    const float len = hit ? dd : (move ? step : 0.f);
+    const float2 pxy = __ffma2_rn(make_float2(len, len), make_float2(s.dx, s.dy), make_float2(s.px, s.py));
+    s.px = pxy.x;
+    s.py = pxy.y;
+    s.pz = fmaf(len, s.dz, s.pz);
+    s.path += len;
+    polar_direction<false>(s.dx, s.dy, s.dz, cpol, sin_from_cos(cpol), d.u2, rx, ry, rz);
+    s.dx = move ? rx : s.dx;
+    s.dy = move ? ry : s.dy;
+    s.dz = move ? rz : s.dz;
+    more = !geo && s.ctr3 < R.ctr_limit;  // at most max_steps steps
+    return more;
+  } else {
+    hit = geo && dd <= s.path;  // arrives inside the time window
+    more = !geo && step <= s.path && s.ctr3 < R.ctr_limit;
+    const float len = geo ? dd : step;
+    const float2 pxy = __ffma2_rn(make_float2(len, len), make_float2(s.dx, s.dy), make_float2(s.px, s.py));
+    s.px = pxy.x;
+    s.py = pxy.y;
+    s.pz = fmaf(len, s.dz, s.pz);
+    s.path -= len;
+    scatter_turn(s.dx, s.dy, s.dz, cpol, sin_from_cos(cpol), d.u2, rx, ry, rz);
+    s.dx = geo ? s.dx : rx;  // a hit keeps its arrival direction
+    s.dy = geo ? s.dy : ry;
+    s.dz = geo ? s.dz : rz;
+    line_of(s);
+    return more && in_reach(s, c.r);
+  }
 }
 
 // Emission (block 0) or step event of one photon.
 template <int MODE, int EM = kEmBasic>
 __device__ __forceinline__ bool photon_event(const DevTables& T, const RunParams& R, const pp_pair* __restrict__ P,
-                                             const PairCtx& c, Photon& s, bool& hit) {
-  if (s.ctr3 < (1u << 8)) {
-    emit_event<MODE, EM>(T, R, P, c, s);
-    return true;
-  }
-  return step_event<MODE>(R, c, s, hit);
+                                             const PairCtx& c, Photon& s, bool& hit, unsigned& steps) {
+  bool more = true, alive;
+  if (s.ctr3 < (1u << 8))
+    alive = emit_event<MODE, EM>(T, R, load_pair(P), s);
+  else
+    alive = step_event<MODE>(R, c, s, hit, more);
+  steps += more ? 1u : 0u;
+  return alive;
 }
 
 // Everything a hit record needs (src/photon_prop_cuda.jl:622,634-641); the
@@ -633,17 +661,19 @@ struct HitValues {
 };
 
 template <int MODE, int EM = kEmBasic>
-__device__ __forceinline__ HitValues hit_values(const DevTables& T, const RunParams& R, const pp_pair* __restrict__ P,
-                                                const PairCtx& c, const Photon& s) {
-  const Draw3 d = emission_uniforms(emission_block(c.seed_lo, c.seed_hi, photon_index(s)));
+__device__ __forceinline__ HitValues hit_values(const DevTables& T, const RunParams& R,
+                                                const pp_pair* __restrict__ pair, const Photon& s) {
+  const PairRec P = load_pair(pair);
+  const Draw3 d = emission_uniforms(emission_block(P.seed_lo, P.seed_hi, photon_index(s)));
   const EmissionFrame f = emission_frame<MODE, EM>(T, P, d);
   HitValues h;
   h.wl = f.wl;
-  emission_direction(f, d.u2, h.d0x, h.d0y, h.d0z);
-  const float3 tg = pair_target(P);
-  h.px = s.px + tg.x;
-  h.py = s.py + tg.y;
-  h.pz = s.pz + tg.z;
+  h.d0x = f.rx;
+  h.d0y = f.ry;
+  h.d0z = f.rz;
+  h.px = s.px + P.tgt_r.x;
+  h.py = s.py + P.tgt_r.y;
+  h.pz = s.pz + P.tgt_r.z;
   h.dist = (MODE == kPhysical) ? path_at_tmax(T, R, f) - s.path : s.path;
   const float x = 1.f / f.wl;
   if (MODE == kCompat) {

@@ -24,22 +24,50 @@ namespace ppd {
 // ---------------------------------------------------------------------------
 // Batched persistent kernel.
 //
-// Each warp owns a ring of kStage staged emissions in shared memory.  When
-// its dead lanes outnumber the staged photons, all 32 lanes take the next
-// photon indices from the warp's chunk (grabbing chunks from the device work
-// queue) and compute 32 emissions together, converged; dead lanes then pick
-// staged photons up with four 16-byte loads.  The step loop that follows
-// is the same straight-line code for every lane.
+// Each warp takes photon chunks from the device work queue and emits 32
+// photons of one pair at a time, converged.  What follows differs by mode:
+//
+// Physical mode: photons end after very different numbers of steps (3.4 on
+// average in the mixed batch), so the warp stages emissions in a ring of
+// kStage photons in shared memory, dead lanes pick staged photons up with
+// four 16-byte loads, and all 32 lanes step together.
+//
+// Compat mode: every photon makes max_steps steps unless it hits, so the 32
+// emitted photons step in lockstep to their end: no ring, no refill, and
+// the lanes of the few that hit idle.
+//
+// Bound by instruction issue (77 % of the issue slots, ALU half-rate pipe
+// 50 %); what counts is instructions per photon.  512 mixed pairs (1.1e8
+// photons): 3.00e9 -> 2.36e9 warp instructions, 3.47 -> 2.85 ms, by testing
+// the reach where a photon stops (in_reach), one emission pass per pair with
+// its record by broadcast, and separate loops for the full warp and for the
+// last photons; 4096 mixed pairs (5.75e9 photons): 171 -> 139 ms; compat
+// mode in lockstep, 100 distances of 2e7 photons with their fits: 175 -> 130
+// ms.  Measured and not kept: the first one or two steps inside the emission
+// pass (fewer loop iterations, but 180 bytes spilled at 64 registers: 3.26 ms).
 constexpr int kStage = 64;  // >= 2 * 32 - 1 staged emissions per warp (power of two)
 
-struct __align__(16) Staged {
-  float px, py, pz, dx, dy, dz, neg_ln2_len, path;
-  uint32_t id_lo, id_hi;
-  int32_t pair;
-  float radius;         // the pair's sphere radius, so that a refill reads
-  uint32_t sc0, sc1;  // shared memory only, and the photon's step stream
-  uint32_t pad[2];
+// The ring holds a photon's 16 words as four arrays of 16-byte words, so that
+// neighbouring lanes read and write neighbouring words (one 64-byte record
+// per photon put the lanes of a store or load on a quarter of the banks):
+//   0: px py pz dx   1: dy dz neg_ln2_len path
+//   2: index lo, the first step's counter word, pair, the pair's sphere radius (a refill reads shared memory only)
+//   3: the step stream's words, a, q
+//
+// A warp's current photon chunk, with a copy of its pair's record, is kept in
+// shared memory too: only the emission pass reads or advances it, so the
+// step loop holds no registers for it.  A pass emits photons of one pair, so
+// it reads the record by broadcast.
+template <int MODE>
+struct __align__(16) WarpArea {
+  float4 ring[4][MODE == kPhysical ? kStage : 1];
+  float4 rec[5];            // the chunk's pp_pair
+  unsigned long long base;  // next photon index of the chunk
+  unsigned left;            // photons left in the chunk
+  int pair;
+  WarpStats stats;
 };
+static_assert(sizeof(pp_pair) == 5 * sizeof(float4), "the record is copied as 16-byte words");
 
 // Compat mode hits often: a photon whose line meets the sphere beyond its
 // step waits in place, pointing at it, until a step reaches it (3.6 % of the
@@ -48,16 +76,6 @@ struct __align__(16) Staged {
 // staged hits together, converged, instead of one or two lanes walking the
 // hit path while the others wait.
 constexpr unsigned kHitStage = 32;
-
-// A warp's current photon chunk (warp-uniform): kept in shared memory, since
-// only the warp's emission pass reads or advances it, so that the step loop
-// holds no registers for it.
-struct WarpChunk {
-  unsigned long long base;  // first photon index of the chunk
-  unsigned next, len;
-  int pair;
-  int done;  // the work queue is exhausted
-};
 struct StagedHit {
   float px, py, pz, dx, dy, dz, path;
   uint32_t id_lo, id_hi;
@@ -72,32 +90,27 @@ template <int MODE, int WARPS, int EM>
 __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / (WARPS * 32))
     batched_kernel(const RunParams R) {
   __shared__ __align__(16) DevTables T;
-  __shared__ Staged stage[WARPS][kStage];
-  __shared__ WarpStats wstats[WARPS];
+  __shared__ WarpArea<MODE> area[WARPS];
   __shared__ StagedHit hstage[MODE == kCompat ? WARPS : 1][kHitStage];
-  __shared__ WarpChunk wchunk[WARPS];
   stage_tables(T, R.tables);
-  if ((threadIdx.x & 31u) == 0) {
-    WarpStats& w0 = wstats[threadIdx.x >> 5];
-    w0.pair = -1;
-    for (int k = 0; k < 6; ++k) w0.v[k] = 0.0;
-    WarpChunk& q = wchunk[threadIdx.x >> 5];
-    q.base = 0;
-    q.next = q.len = 0;
-    q.pair = 0;
-    q.done = 0;
+  const unsigned lane = threadIdx.x & 31u;
+  WarpArea<MODE>* wa = &area[threadIdx.x >> 5];
+  if (lane == 0) {
+    wa->stats.pair = -1;
+    for (int k = 0; k < 6; ++k) wa->stats.v[k] = 0.0;
+    wa->left = 0;
+    wa->pair = 0;
   }
   __syncthreads();
 
-  const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;
-  Staged* ring = stage[threadIdx.x >> 5];
-  WarpStats* ws = &wstats[threadIdx.x >> 5];
+  WarpStats* ws = &wa->stats;
   StagedHit* hst = hstage[MODE == kCompat ? (threadIdx.x >> 5) : 0];
-  unsigned h_count = 0;  // staged hits (compat mode), warp-uniform
+  unsigned h_count = 0;  // staged hits, warp-uniform
   const unsigned long long total_chunks = R.chunk_offsets[R.n_pairs];
   // records staged hits 0..n-1 (n warp-uniform), one per lane
   auto record_staged = [&](unsigned n) {
+    __syncwarp();
     if (lane < n) {
       const StagedHit& g = hst[lane];
       Photon p;
@@ -112,146 +125,14 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
       p.id_lo = g.id_lo;
       p.ctr3 = g.id_hi;  // block 0: the index's top bits only
       p.sc0 = p.sc1 = 0u;
-      const PairCtx pc = load_pair_ctx(R.pairs + g.pair, g.pair);
-      const HitValues h = hit_values<MODE, EM>(T, R, R.pairs + g.pair, pc, p);
+      const PairCtx pc{0.f, g.pair};
+      const HitValues h = hit_values<MODE, EM>(T, R, R.pairs + g.pair, p);
       record_hit_cached(R, ws, pc, p, h);
     }
     __syncwarp();
   };
-
-  // warp-uniform state: the ring (the current chunk is in shared memory)
-  WarpChunk* wq = &wchunk[threadIdx.x >> 5];
-  unsigned r_head = 0, r_count = 0;
-
-  // lane state
-  bool alive = false;
-  Photon s;
-  s.id_lo = 0;
-  s.ctr3 = 1u << 8;
-  s.sc0 = s.sc1 = 0u;
-  s.px = s.py = s.pz = s.dx = s.dy = s.path = s.neg_ln2_len = 0.f;
-  s.dz = 1.f;
-  // the lane's pair: radius and index (the seed, which only a hit's emission
-  // replay needs, is read from the pair record then)
-  PairCtx c;
-  c.r = 0.f;
-  c.seed_lo = c.seed_hi = 0u;
-  c.index = 0;
-  unsigned steps = 0;
-
-  for (;;) {
-    const unsigned need = __ballot_sync(kFull, !alive);
-    const unsigned n_need = __popc(need);
-    if (r_count < n_need && !wq->done) {
-      unsigned long long c_base = wq->base;
-      unsigned c_next = wq->next, c_len = wq->len;
-      int c_pair = wq->pair;
-      bool queue_done = false;
-      // give every lane the next photon index of the queue
-      bool have = false;
-      unsigned long long pid = 0;
-      int ppair = 0;
-      unsigned filled = 0;
-      while (filled < 32u) {
-        if (c_next >= c_len) {
-          unsigned long long cid = 0, start = 0, end = 0;
-          int p = 0;
-          if (lane == 0) {
-            cid = atomicAdd(R.queue, 1ull);
-            if (cid < total_chunks) {
-              int lo = 0, hi = (int)R.n_pairs - 1;  // last pair whose first chunk <= cid
-              while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (R.chunk_offsets[mid] <= cid) lo = mid; else hi = mid - 1;
-              }
-              p = lo;
-              if (EM == kEmBasic && R.pairs[p].emitter == PP_EMITTER_CASCADE)
-                atomicOr(R.counters + 2, 4ull);  // a cascade pair in a launch without PP_OPT_CASCADE
-              start = (cid - R.chunk_offsets[p]) * (unsigned long long)R.chunk;
-              end = min(start + (unsigned long long)R.chunk, (unsigned long long)R.pairs[p].n_photons);
-            }
-          }
-          cid = __shfl_sync(kFull, cid, 0);
-          if (cid >= total_chunks) {
-            queue_done = true;
-            break;
-          }
-          c_pair = __shfl_sync(kFull, p, 0);
-          if (c_pair != ws->pair) {  // the warp's statistics cache follows its chunk
-            if (lane == 0) {
-              flush_warp_stats(R.stats, ws);
-              ws->pair = c_pair;
-            }
-            __syncwarp();
-          }
-          c_base = __shfl_sync(kFull, start, 0);
-          c_len = (unsigned)(__shfl_sync(kFull, end, 0) - c_base);
-          c_next = 0;
-        }
-        const unsigned take = min(32u - filled, c_len - c_next);
-        if (lane >= filled && lane < filled + take) {
-          have = true;
-          pid = c_base + (c_next + (lane - filled));
-          ppair = c_pair;
-        }
-        c_next += take;
-        filled += take;
-      }
-      if (lane == 0) {
-        wq->base = c_base;
-        wq->next = c_next;
-        wq->len = c_len;
-        wq->pair = c_pair;
-        wq->done = queue_done;
-      }
-      if (have) {
-        const pp_pair* P = R.pairs + ppair;
-        const PairCtx pc = load_pair_ctx(P, ppair);
-        Photon e;
-        set_photon(e, pid);
-        emit_event<MODE, EM>(T, R, P, pc, e);
-        float4* dst = reinterpret_cast<float4*>(ring + ((r_head + r_count + lane) & (kStage - 1)));
-        dst[0] = make_float4(e.px, e.py, e.pz, e.dx);
-        dst[1] = make_float4(e.dy, e.dz, e.neg_ln2_len, e.path);
-        dst[2] = make_float4(__uint_as_float((uint32_t)pid), __uint_as_float((uint32_t)(pid >> 32)),
-                             __int_as_float(ppair), pc.r);
-        dst[3] = make_float4(__uint_as_float(e.sc0), __uint_as_float(e.sc1), 0.f, 0.f);
-      }
-      r_count += filled;
-      __syncwarp();
-    }
-    if (!alive) {
-      const unsigned rank = __popc(need & lt_mask);
-      if (rank < r_count) {
-        const float4* src = reinterpret_cast<const float4*>(ring + ((r_head + rank) & (kStage - 1)));
-        const float4 a = src[0], b = src[1], d = src[2], e = src[3];
-        s.px = a.x;
-        s.py = a.y;
-        s.pz = a.z;
-        s.dx = a.w;
-        s.dy = b.x;
-        s.dz = b.y;
-        s.neg_ln2_len = b.z;
-        s.path = b.w;
-        s.id_lo = __float_as_uint(d.x);
-        s.ctr3 = __float_as_uint(d.y) | (1u << 8);  // index bits 32..39, step 0
-        c.index = __float_as_int(d.z);
-        c.r = d.w;
-        s.sc0 = __float_as_uint(e.x);
-        s.sc1 = __float_as_uint(e.y);
-        alive = true;
-      }
-    }
-    const unsigned took = min(n_need, r_count);
-    r_head += took;
-    r_count -= took;
-    __syncwarp();
-    if (need == kFull && took == 0u) break;  // every lane was idle and none took a photon
-    bool hit = false;
-    if (alive) {
-      ++steps;
-      alive = step_event<MODE>(R, c, s, hit);
-    }
+  // takes the hits of a step (all lanes call)
+  auto take_hits = [&](bool hit, const Photon& p, const PairCtx& c) {
     if (MODE == kCompat) {
       const unsigned hm = __ballot_sync(kFull, hit);
       if (hm) {
@@ -262,34 +143,176 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
         }
         if (hit) {
           StagedHit& g = hst[h_count + __popc(hm & lt_mask)];
-          g.px = s.px;
-          g.py = s.py;
-          g.pz = s.pz;
-          g.dx = s.dx;
-          g.dy = s.dy;
-          g.dz = s.dz;
-          g.path = s.path;
-          g.id_lo = s.id_lo;
-          g.id_hi = s.ctr3 & 0xFFu;
+          g.px = p.px;
+          g.py = p.py;
+          g.pz = p.pz;
+          g.dx = p.dx;
+          g.dy = p.dy;
+          g.dz = p.dz;
+          g.path = p.path;
+          g.id_lo = p.id_lo;
+          g.id_hi = p.ctr3 & 0xFFu;
           g.pair = c.index;
         }
         h_count += nh;
-        __syncwarp();
-        if (h_count == kHitStage) {
-          record_staged(kHitStage);
-          h_count = 0;
-        }
       }
     } else if (__any_sync(kFull, hit)) {
       if (hit) {
-        const PairCtx pc = load_pair_ctx(R.pairs + c.index, c.index);
-        const HitValues h = hit_values<MODE, EM>(T, R, R.pairs + c.index, pc, s);
-        record_hit_cached(R, ws, pc, s, h);
+        const HitValues h = hit_values<MODE, EM>(T, R, R.pairs + c.index, p);
+        record_hit_cached(R, ws, c, p, h);
       }
     }
+  };
+  // the warp's next chunk of the queue, its pair's record and statistics
+  // cache; false when the queue is exhausted
+  auto fetch = [&]() {
+    int p = -1;
+    if (lane == 0) {
+      const unsigned long long cid = atomicAdd(R.queue, 1ull);
+      if (cid < total_chunks) {
+        int hi = (int)R.n_pairs - 1;  // last pair whose first chunk <= cid
+        p = 0;
+        while (p < hi) {
+          const int mid = (p + hi + 1) >> 1;
+          if (R.chunk_offsets[mid] <= cid) p = mid; else hi = mid - 1;
+        }
+        const unsigned long long start = (cid - R.chunk_offsets[p]) * (unsigned long long)R.chunk;
+        wa->base = start;
+        wa->left = (unsigned)min((unsigned long long)R.chunk, (unsigned long long)R.pairs[p].n_photons - start);
+        wa->pair = p;
+        if (EM == kEmBasic && R.pairs[p].emitter == PP_EMITTER_CASCADE)
+          atomicOr(R.counters + 2, 4ull);  // a cascade pair in a launch without PP_OPT_CASCADE
+        if (p != ws->pair) {               // the warp's statistics cache follows its chunk
+          flush_warp_stats(R.stats, ws);
+          ws->pair = p;
+        }
+      }
+    }
+    p = __shfl_sync(kFull, p, 0);
+    if (p >= 0 && lane < 5u) wa->rec[lane] = __ldg(reinterpret_cast<const float4*>(R.pairs + p) + lane);
+    __syncwarp();
+    return p >= 0;
+  };
+  // emits the chunk's next photons, one per lane (lanes past its end emit as
+  // well, and drop it); returns whether the lane has one that is in reach
+  unsigned steps = 0;  // beyond the photons' first ones, which the set-up kernel has counted
+  auto emit = [&](Photon& e, PairCtx& c) {
+    const unsigned left = wa->left, n = min(32u, left);
+    const uint64_t base = wa->base;
+    c.index = wa->pair;
+    __syncwarp();
+    wa->base = base + n;  // by every lane: the same values
+    wa->left = left - n;
+    set_photon(e, base + lane);
+    const PairRec P = staged_pair(wa->rec);
+    c.r = P.tgt_r.w;
+    const bool near = emit_event<MODE, EM>(T, R, P, e);
+    return near && lane < n;
+  };
+
+  if constexpr (MODE == kCompat) {
+    for (;;) {
+      if (wa->left == 0u && !fetch()) break;
+      Photon s;
+      PairCtx c;
+      bool alive = emit(s, c);
+      do {
+        bool hit, more;
+        step_event<MODE>(R, c, s, hit, more);
+        more = more && alive;
+        take_hits(hit && alive, s, c);
+        steps += more ? 1u : 0u;
+        alive = more;
+      } while (__any_sync(kFull, alive));
+    }
+  } else {
+    // warp-uniform state of the ring, and the lane's photon and pair (radius
+    // and index: the rest of its record, which only a hit's emission replay
+    // needs, is read then)
+    unsigned r_head = 0, r_count = 0;
+    bool alive = false;
+    Photon s;
+    s.id_lo = 0;
+    s.ctr3 = 1u << 8;
+    s.sc0 = s.sc1 = 0u;
+    s.px = s.py = s.pz = s.dx = s.dy = s.path = s.neg_ln2_len = 0.f;
+    s.dz = 1.f;
+    s.a = s.q = 0.f;
+    PairCtx c;
+    c.r = 0.f;
+    c.index = 0;
+    // the lane's next photon: the ring's entry of its rank among the lanes in need
+    auto take_staged = [&](unsigned need) {
+      const unsigned slot = (r_head + __popc(need & lt_mask)) & (kStage - 1);
+      const float4 a = wa->ring[0][slot], b = wa->ring[1][slot], d = wa->ring[2][slot], e = wa->ring[3][slot];
+      s.px = a.x;
+      s.py = a.y;
+      s.pz = a.z;
+      s.dx = a.w;
+      s.dy = b.x;
+      s.dz = b.y;
+      s.neg_ln2_len = b.z;
+      s.path = b.w;
+      s.id_lo = __float_as_uint(d.x);
+      s.ctr3 = __float_as_uint(d.y);
+      c.index = __float_as_int(d.z);
+      c.r = d.w;
+      s.sc0 = __float_as_uint(e.x);
+      s.sc1 = __float_as_uint(e.y);
+      s.a = e.z;
+      s.q = e.w;
+    };
+    // While the ring can fill every lane in need, all 32 lanes step together
+    // and nothing else is tested.
+    for (;;) {
+      const unsigned need = __ballot_sync(kFull, !alive), n_need = __popc(need);
+      // emission passes, until the ring can (photons that start out of reach
+      // are not staged) or the queue is exhausted
+      while (r_count < n_need) {
+        if (wa->left == 0u && !fetch()) break;
+        Photon e;
+        PairCtx ec;
+        const bool near = emit(e, ec);
+        const unsigned keep = __ballot_sync(kFull, near);
+        if (near) {
+          const unsigned slot = (r_head + r_count + __popc(keep & lt_mask)) & (kStage - 1);
+          wa->ring[0][slot] = make_float4(e.px, e.py, e.pz, e.dx);
+          wa->ring[1][slot] = make_float4(e.dy, e.dz, e.neg_ln2_len, e.path);
+          wa->ring[2][slot] = make_float4(__uint_as_float(e.id_lo), __uint_as_float(e.ctr3),
+                                          __int_as_float(ec.index), ec.r);
+          wa->ring[3][slot] = make_float4(__uint_as_float(e.sc0), __uint_as_float(e.sc1), e.a, e.q);
+        }
+        r_count += __popc(keep);
+        __syncwarp();
+      }
+      if (r_count < n_need) break;
+      if (!alive) take_staged(need);
+      r_head += n_need;
+      r_count -= n_need;
+      bool hit, more;
+      alive = step_event<MODE>(R, c, s, hit, more);
+      steps += more ? 1u : 0u;
+      take_hits(hit, s, c);
+    }
+    // The ring's last photons, then ever fewer lanes.
+    for (;;) {
+      const unsigned need = __ballot_sync(kFull, !alive);
+      if (!alive && __popc(need & lt_mask) < r_count) {
+        take_staged(need);
+        alive = true;
+      }
+      if (need == kFull && r_count == 0u) break;  // every lane was idle and none took a photon
+      const unsigned took = min((unsigned)__popc(need), r_count);
+      r_head += took;
+      r_count -= took;
+      bool hit = false, more = false;
+      if (alive) alive = step_event<MODE>(R, c, s, hit, more);
+      steps += more ? 1u : 0u;
+      take_hits(hit, s, c);
+    }
   }
-  __syncwarp();
   if (MODE == kCompat && h_count > 0u) record_staged(h_count);
+  __syncwarp();
   if (lane == 0) flush_warp_stats(R.stats, ws);
   // photon-step count for the roofline
   unsigned long long st = steps;
@@ -306,7 +329,7 @@ __global__ void __launch_bounds__(512) plain_kernel(const RunParams R, const pp_
   __shared__ __align__(16) DevTables T;
   stage_tables(T, R.tables);
   __syncthreads();
-  const PairCtx c = load_pair_ctx(pair_ptr, pair_index);
+  const PairCtx c{pair_ptr->radius, pair_index};
   const unsigned long long n = (unsigned long long)pair_ptr->n_photons;
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   unsigned steps = 0;
@@ -319,10 +342,9 @@ __global__ void __launch_bounds__(512) plain_kernel(const RunParams R, const pp_
     bool alive = true;
     while (alive) {
       bool hit = false;
-      steps += (s.ctr3 >= (1u << 8));
-      alive = photon_event<MODE, EM>(T, R, pair_ptr, c, s, hit);
+      alive = photon_event<MODE, EM>(T, R, pair_ptr, c, s, hit, steps);
       if (hit) {
-        const HitValues h = hit_values<MODE, EM>(T, R, pair_ptr, c, s);
+        const HitValues h = hit_values<MODE, EM>(T, R, pair_ptr, s);
         record_hit(R, c, s, h, 0);
       }
     }
@@ -349,7 +371,7 @@ __global__ void __launch_bounds__(1024) stacks_kernel(const RunParams R, const p
   const int ix_offset = (int)blockIdx.x * stack_len + 1;  // 1-based, as in the reference
   if (threadIdx.x == 0) cursor = ix_offset;
   __syncthreads();
-  const PairCtx c = load_pair_ctx(pair_ptr, 0);
+  const PairCtx c{pair_ptr->radius, 0};
   const int safe_margin = max(0, (int)blockDim.x - 32);
   const unsigned long long G = (unsigned long long)gridDim.x * blockDim.x;
   const unsigned long long g = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -364,10 +386,9 @@ __global__ void __launch_bounds__(1024) stacks_kernel(const RunParams R, const p
     bool alive = true;
     while (alive) {
       bool hit = false;
-      steps += (s.ctr3 >= (1u << 8));
-      alive = photon_event<MODE, kEmCascade>(T, R, pair_ptr, c, s, hit);
+      alive = photon_event<MODE, kEmCascade>(T, R, pair_ptr, c, s, hit, steps);
       if (hit) {
-        const HitValues h = hit_values<MODE, kEmCascade>(T, R, pair_ptr, c, s);
+        const HitValues h = hit_values<MODE, kEmCascade>(T, R, pair_ptr, s);
         const int idx = atomicAdd(&cursor, 1);  // 1-based slot
         if (idx < ix_offset + stack_len) {
           const int j = idx - 1;
@@ -439,9 +460,21 @@ __global__ void __launch_bounds__(1024) chunk_scan_kernel(const pp_pair* __restr
   if (t == 0) {
     queue[0] = 0ull;
     counters[0] = 0ull;
-    counters[1] = 0ull;
     counters[2] = 0ull;
     counters[3] = 0ull;
+  }
+  // counters[1] starts as the photons' first steps; the batched kernel adds the others
+  unsigned long long photons = 0;
+  for (int64_t i = b; i < e; ++i) photons += (unsigned long long)max((long long)pairs[i].n_photons, 0ll);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) photons += __shfl_xor_sync(kFull, photons, o);
+  __syncthreads();
+  if (lane == 0) warp_sums[warp] = photons;
+  __syncthreads();
+  if (t == 0) {
+    unsigned long long sum = 0;
+    for (unsigned w = 0; w < (blockDim.x >> 5); ++w) sum += warp_sums[w];
+    counters[1] = sum;
   }
 }
 
@@ -492,13 +525,7 @@ __global__ void eval_kernel(int op, const double* __restrict__ in, double* __res
     }
     case 2: {
       const float g = (float)in[2 * i];
-      HG h;
-      h.iso = (g == 0.f);
-      h.two_g = 2.f * g;
-      h.one_m_g = 1.f - g;
-      h.a = 1.f - g * g;
-      h.one_p_g2 = 1.f + g * g;
-      h.inv_2g = h.iso ? 0.f : 1.f / (2.f * g);
+      const HG h = make_hg(g);
       out[i] = (double)hg_costheta(h, (float)in[2 * i + 1]);
       break;
     }
@@ -585,7 +612,6 @@ __global__ void __launch_bounds__(256, 4) peak_step_kernel(const RunParams R, in
                                                            unsigned long long* __restrict__ out) {
   PairCtx c;
   c.r = 0.21f;
-  c.seed_lo = c.seed_hi = 0u;
   c.index = 0;
   Photon s;
   s.sc0 = 0x9E3779B9u * (blockIdx.x + 1u) ^ threadIdx.x;
@@ -601,12 +627,14 @@ __global__ void __launch_bounds__(256, 4) peak_step_kernel(const RunParams R, in
   s.path = 1e30f;
   s.neg_ln2_len = -kLn2 * 30.f;
   s.ctr3 = ctr_word(id, 1u);
-  unsigned live = 0;
+  line_of(s);
+  unsigned live = 0, steps = 0;
   for (int i = 0; i < iters; ++i) {
-    bool hit = false;
-    live += step_event<kPhysical>(R, c, s, hit) ? 1u : 0u;
+    bool hit, more;
+    live += step_event<kPhysical>(R, c, s, hit, more) ? 1u : 0u;
+    steps += more ? 1u : 0u;
   }
-  if (s.px == 1.2345f && s.dz == 0.5f && live == 7u) out[1] = 1ull;
+  if (s.px == 1.2345f && s.dz == 0.5f && live + steps == 7u) out[1] = 1ull;
   if ((threadIdx.x & 31u) == 0) atomicAdd(out, 32ull * (unsigned long long)iters);
 }
 
@@ -637,13 +665,7 @@ static __host__ ppd::RunParams to_params(const LaunchArgs& a) {
   R.inv_bin_width = a.opts.hist_bin_width > 0.f ? 1.f / a.opts.hist_bin_width : 0.f;
   R.hist_bins = a.opts.hist_bins;
   R.flags = a.opts.flags;
-  const float g = a.opts.g;
-  R.hg.iso = (g == 0.f);
-  R.hg.two_g = 2.f * g;
-  R.hg.one_m_g = 1.f - g;
-  R.hg.a = 1.f - g * g;
-  R.hg.one_p_g2 = 1.f + g * g;
-  R.hg.inv_2g = R.hg.iso ? 0.f : 1.f / (2.f * g);
+  R.hg = ppd::make_hg(a.opts.g);
   return R;
 }
 
@@ -667,6 +689,8 @@ void fill_dev_tables(void* host_tables, const double coeffs[11], const float* kn
   t->sca2 = (float)coeffs[6];
   t->n_knots = n_knots;
   for (int i = 0; i < n_knots; ++i) t->knots[i] = knots[i];
+  t->n_cells = n_knots > 1 ? n_knots - 1 : 1;
+  if (n_knots == 1) t->knots[1] = t->knots[0];
   t->n_abs = n_abs;
   for (int i = 0; i < n_abs; ++i) {
     t->abs_wl[i] = abs_wl[i];
