@@ -3,7 +3,7 @@
 // A context holds the device-resident physics tables, a stream, the device
 // buffers of the host-buffer entry points, the work-queue scratch of the
 // batched kernel, the tuned launch shape per mode and a small cache of
-// instantiated CUDA graphs (scan -> batched kernel -> finalise) keyed by the
+// instantiated CUDA graphs (set-up -> batched kernel) keyed by the
 // call's shapes and buffers.
 #include <cuda_runtime.h>
 
@@ -26,8 +26,12 @@ static std::atomic<uint64_t> g_launches{0};
 // Launches enqueued while a thread captures a graph run only when the graph
 // is launched; they are counted then.
 static thread_local bool g_capturing = false;
+static thread_local uint64_t g_captured = 0;  // kernels of the graph being captured
 void count_launches(uint64_t n) {
-  if (!g_capturing) g_launches.fetch_add(n, std::memory_order_relaxed);
+  if (g_capturing)
+    g_captured += n;
+  else
+    g_launches.fetch_add(n, std::memory_order_relaxed);
 }
 }  // namespace pp
 
@@ -88,11 +92,12 @@ struct GraphKey {
 struct GraphEntry {
   GraphKey key;
   cudaGraphExec_t exec = nullptr;
+  uint64_t kernels = 0;
   uint64_t last_use = 0;
 };
 
 constexpr int kGraphCache = 4;
-constexpr int kKernelsPerBatch = 3;  // scan, batched, finalise
+bool normalizes(const pp_run_opts& o) { return (o.flags & PP_OPT_NORMALIZE) && o.hist_bins > 0; }
 
 }  // namespace
 
@@ -211,17 +216,14 @@ void resolve_launch(pp_ctx* c, const pp_run_opts& o, int& grid, int& block, uint
   chunk = (uint32_t)(o.chunk_photons > 0 ? o.chunk_photons : c->tuned_chunk[m]);
 }
 
-// memset stats/hist, scan (resets queue and counters), batched kernel, finalise.
+// set-up (zeroed outputs, queue, counters), batched kernel, normalisation.
 cudaError_t enqueue_batched(pp_ctx* c, const pp::LaunchArgs& a, int grid, int block, cudaStream_t s) {
   cudaError_t e;
-  if (a.stats && (e = cudaMemsetAsync(a.stats, 0, (size_t)a.n_pairs * PP_STATS * sizeof(double), s))) return e;
-  if (a.hist && a.opts.hist_bins > 0 &&
-      (e = cudaMemsetAsync(a.hist, 0, (size_t)a.n_pairs * a.opts.hist_bins * sizeof(double), s)))
-    return e;
-  if ((e = pp::launch_chunk_scan(a, s))) return e;
+  if ((e = pp::launch_setup(a, c->sm_count, s))) return e;
   if ((e = pp::launch_batched(a, grid, block, s))) return e;
-  return pp::launch_finalize(a.pairs, a.n_pairs, a.stats, a.hist, a.opts.hist_bins,
-                             (a.opts.flags & PP_OPT_NORMALIZE) ? 1 : 0, c->sm_count, s);
+  if (a.hist && normalizes(a.opts))
+    return pp::launch_normalize(a.pairs, a.n_pairs, a.hist, a.opts.hist_bins, c->sm_count, s);
+  return cudaSuccess;
 }
 
 // Replays a cached graph for this key or captures a new one.  Streams that
@@ -243,7 +245,7 @@ cudaError_t run_batched(pp_ctx* c, const pp::LaunchArgs& a, cudaStream_t s, bool
   k.stats = b.stats;
   k.hist = b.hist;
   k.stream = s;
-  k.offsets = b.chunk_offsets;
+  k.offsets = b.granule_offsets;
   k.queue = b.queue;
   k.grid = grid;
   k.block = block;
@@ -252,7 +254,7 @@ cudaError_t run_batched(pp_ctx* c, const pp::LaunchArgs& a, cudaStream_t s, bool
   for (auto& g : c->graphs) {
     if (g.exec && g.key == k) {
       g.last_use = ++c->graph_clock;
-      pp::count_launches(kKernelsPerBatch);
+      pp::count_launches(g.kernels);
       return cudaGraphLaunch(g.exec, s);
     }
   }
@@ -260,8 +262,10 @@ cudaError_t run_batched(pp_ctx* c, const pp::LaunchArgs& a, cudaStream_t s, bool
   cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
   if (e) return e;
   pp::g_capturing = true;
+  pp::g_captured = 0;
   cudaError_t le = enqueue_batched(c, b, grid, block, s);
   pp::g_capturing = false;
+  const uint64_t kernels = pp::g_captured;
   e = cudaStreamEndCapture(s, &graph);
   if (le) {
     if (graph) cudaGraphDestroy(graph);
@@ -286,7 +290,8 @@ cudaError_t run_batched(pp_ctx* c, const pp::LaunchArgs& a, cudaStream_t s, bool
   }
   slot->key = k;
   slot->last_use = ++c->graph_clock;
-  pp::count_launches(kKernelsPerBatch);
+  slot->kernels = kernels;
+  pp::count_launches(kernels);
   return cudaGraphLaunch(slot->exec, s);
 }
 
@@ -515,7 +520,7 @@ pp_status pp_propagate_device(pp_ctx* c, const pp_pair* d_pairs, int64_t n_pairs
   pp::LaunchArgs a = base_args(c, opts);
   a.pairs = d_pairs;
   a.n_pairs = n_pairs;
-  a.chunk_offsets = static_cast<unsigned long long*>(c->offsets.p);
+  a.granule_offsets = static_cast<unsigned long long*>(c->offsets.p);
   a.queue = static_cast<unsigned long long*>(c->queue.p);
   a.hits = d_hits;
   a.hit_cap = (unsigned long long)cap;
@@ -557,7 +562,7 @@ pp_status pp_propagate(pp_ctx* c, const pp_pair* pairs, int64_t n_pairs, const p
   pp::LaunchArgs a = base_args(c, opts);
   a.pairs = static_cast<const pp_pair*>(c->pairs.p);
   a.n_pairs = n_pairs;
-  a.chunk_offsets = static_cast<unsigned long long*>(c->offsets.p);
+  a.granule_offsets = static_cast<unsigned long long*>(c->offsets.p);
   a.queue = static_cast<unsigned long long*>(c->queue.p);
   a.hits = static_cast<pp_hit*>(c->hits.p);
   a.hit_cap = (unsigned long long)cap;
@@ -620,13 +625,9 @@ pp_status pp_propagate_plain_device(pp_ctx* c, const pp_pair* d_pair, const pp_p
   const long long need = (h_pair->n_photons + block - 1) / block;
   int grid = (int)std::min<long long>((long long)c->sm_count * bps, std::max<long long>(need, 1));
   cudaError_t e;
-  if ((e = cudaMemsetAsync(d_stats, 0, PP_STATS * sizeof(double), s))) return c->cuda_fail(e, "memset");
-  if (a.hist && (e = cudaMemsetAsync(a.hist, 0, (size_t)opts->hist_bins * sizeof(double), s)))
-    return c->cuda_fail(e, "memset");
-  if ((e = pp::launch_reset_counters(a.counters, s)) ||
-      (e = pp::launch_plain(a, d_pair, (int)pair_index, grid, block, s)) ||
-      (e = pp::launch_finalize(d_pair, 1, d_stats, a.hist, opts->hist_bins, (opts->flags & PP_OPT_NORMALIZE) ? 1 : 0,
-                               c->sm_count, s)))
+  if ((e = pp::launch_setup(a, c->sm_count, s)) || (e = pp::launch_plain(a, d_pair, (int)pair_index, grid, block, s)) ||
+      (a.hist && normalizes(*opts) &&
+       (e = pp::launch_normalize(d_pair, 1, a.hist, opts->hist_bins, c->sm_count, s))))
     return c->cuda_fail(e, "plain launch");
   return PP_OK;
 }
@@ -731,7 +732,7 @@ pp_status pp_cuda_propagate_photons(pp_ctx* c, float* pos, float* dir, float* wl
   a.counters = static_cast<unsigned long long*>(c->counters.p);
   const long long G = (long long)n_blocks * threads;
   const long long per_thread = (st_pair->n_photons + G - 1) / G;  // cld(photons, grid*block), :288
-  if ((e = pp::launch_reset_counters(a.counters, s)) ||
+  if ((e = pp::launch_setup(a, c->sm_count, s)) ||
       (e = pp::launch_stacks(a, a.pairs, pos, dir, wl, dist, sp, nsim, stack_len, n_blocks, threads, per_thread, s)))
     return c->cuda_fail(e, "stacks launch");
   // the reference call is synchronous (CUDA.jl launches block on copy-back)
@@ -850,7 +851,7 @@ static pp_status pilot_estimate(pp_ctx* c, const pp_pair* pairs, int64_t n_pairs
   pp::LaunchArgs a = base_args(c, &po);
   a.pairs = static_cast<const pp_pair*>(c->pilot.p);
   a.n_pairs = n_pairs;
-  a.chunk_offsets = static_cast<unsigned long long*>(c->offsets.p);
+  a.granule_offsets = static_cast<unsigned long long*>(c->offsets.p);
   a.queue = static_cast<unsigned long long*>(c->queue.p);
   a.hits = static_cast<pp_hit*>(c->hits.p);
   a.hit_cap = 0;
@@ -946,7 +947,7 @@ pp_status pp_propagate_fit(pp_ctx* c, const pp_pair* pairs, int64_t n_pairs, con
       a.pairs = d_pairs + start;
       a.n_pairs = end - start;
       a.pair_base = (uint32_t)start;
-      a.chunk_offsets = static_cast<unsigned long long*>(c->offsets.p);
+      a.granule_offsets = static_cast<unsigned long long*>(c->offsets.p);
       a.queue = static_cast<unsigned long long*>(c->queue.p);
       a.hits = static_cast<pp_hit*>(c->hits.p);
       a.hit_cap = (unsigned long long)cap;
@@ -1184,7 +1185,7 @@ pp_status propagate_with_scratch(pp_ctx* c, const pp_pair* d_pairs, int64_t n_pa
   a.pairs = d_pairs;
   a.n_pairs = n_pairs;
   a.queue = d_queue;
-  a.chunk_offsets = d_offsets;
+  a.granule_offsets = d_offsets;
   a.chunk = chunk;
   a.hits = static_cast<pp_hit*>(d_hits);
   a.hit_cap = (unsigned long long)cap;
@@ -1268,7 +1269,7 @@ extern "C" pp_status pp_propagate_device_noalloc(pp_ctx* c, const pp_pair* d_pai
   a.pairs = d_pairs;
   a.n_pairs = n_pairs;
   a.queue = scratch;
-  a.chunk_offsets = scratch + kNoallocQueueWords;
+  a.granule_offsets = scratch + kNoallocQueueWords;
   a.chunk = chunk;
   a.hits = d_hits;
   a.hit_cap = (unsigned long long)cap;

@@ -337,9 +337,9 @@ __device__ __forceinline__ void rotate_to_axis(float ox, float oy, float oz, flo
 struct RunParams {
   const pp_pair* __restrict__ pairs;
   int64_t n_pairs;
-  const unsigned long long* __restrict__ chunk_offsets;  // [n_pairs + 1]
-  unsigned long long* __restrict__ queue;                // [0]: next chunk
-  uint32_t chunk;
+  const unsigned long long* __restrict__ granule_offsets;  // [n_pairs + 1] first 32-photon granule of each pair
+  unsigned long long* __restrict__ queue;                  // [0]: next granule
+  uint32_t max_run;  // granules a warp takes at once, at most
   uint32_t pair_base;  // added to the pair index written into hits
   pp_hit* __restrict__ hits;
   unsigned long long hit_cap;

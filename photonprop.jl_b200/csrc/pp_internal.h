@@ -27,9 +27,9 @@ struct Range {
 struct LaunchArgs {
   const pp_pair* pairs;
   int64_t n_pairs;
-  unsigned long long* chunk_offsets;  // [n_pairs + 1] scratch
-  unsigned long long* queue;          // [1] scratch
-  uint32_t chunk;
+  unsigned long long* granule_offsets;  // [n_pairs + 1] scratch
+  unsigned long long* queue;            // [1] scratch
+  uint32_t chunk;                       // photons a warp takes from the queue at once, at most
   pp_hit* hits;
   unsigned long long hit_cap;
   unsigned long long* counters;  // [4]
@@ -52,16 +52,16 @@ void fill_dev_tables(void* host_tables, const double coeffs[11], const float* kn
 void set_cascade_tables(void* host_tables, const float* d_casc, double gmin, double gmax);
 void get_dev_knots(const void* host_tables, float* out, int* n);
 
-cudaError_t launch_chunk_scan(const LaunchArgs& a, cudaStream_t s);
-cudaError_t launch_reset_counters(unsigned long long* counters, cudaStream_t s);
+// zeroed statistics and histograms, counters and work queue of a launch
+// (granule_offsets == NULL: no queue)
+cudaError_t launch_setup(const LaunchArgs& a, int sm_count, cudaStream_t s);
 cudaError_t launch_batched(const LaunchArgs& a, int grid, int block, cudaStream_t s);
 cudaError_t launch_plain(const LaunchArgs& a, const pp_pair* d_pair, int pair_index, int grid, int block,
                          cudaStream_t s);
 cudaError_t launch_stacks(const LaunchArgs& a, const pp_pair* d_pair, float* pos, float* dir, float* wl,
                           float* dist, int32_t* sp, int64_t* nsim, int stack_len, int grid, int block,
                           long long per_thread, cudaStream_t s);
-cudaError_t launch_finalize(const pp_pair* pairs, int64_t n, double* stats, double* hist, int bins, int normalize,
-                            int sm_count, cudaStream_t s);
+cudaError_t launch_normalize(const pp_pair* pairs, int64_t n, double* hist, int bins, int sm_count, cudaStream_t s);
 cudaError_t launch_eval(int op, const double* in, double* out, int64_t n, const void* tables, cudaStream_t s);
 int batched_max_blocks_per_sm(int mode, int block, bool cascade);
 int plain_max_blocks_per_sm(int mode, int block);

@@ -1,6 +1,6 @@
 // Kernels of the photon-propagation hot path (sm_100a).
 //
-//  batched_kernel  persistent: each warp pulls photon chunks of any pair from a
+//  batched_kernel  persistent: each warp pulls runs of photons of any pair from a
 //                  device work queue and refills a lane as soon as its photon
 //                  ends, so lanes never idle behind a long-lived photon and
 //                  thousands of uneven pairs run in one launch.
@@ -9,8 +9,9 @@
 //                  thread loop (src/photon_prop_cuda.jl:301-380).
 //  stacks_kernel   cuda_propagate_photons! with the reference's output layout
 //                  (per-block hit stacks, src/photon_prop_cuda.jl:262-386).
-//  chunk_scan_kernel / finalize_kernel   work-queue set-up and FP64
-//                  normalisation.
+//  setup_kernel, fill_kernel   zeroed statistics and histograms, counters,
+//                  work queue.
+//  normalize_kernel  histograms per photon (PP_OPT_NORMALIZE).
 //  eval_kernel     device helpers on test inputs.
 //  peak kernels    FP32 / MUFU / INT issue microbenchmarks for the roofline.
 #include <cooperative_groups.h>
@@ -24,8 +25,10 @@ namespace ppd {
 // ---------------------------------------------------------------------------
 // Batched persistent kernel.
 //
-// Each warp takes photon chunks from the device work queue and emits 32
-// photons of one pair at a time, converged.  What follows differs by mode:
+// The work queue is one row of granules of 32 photons over all pairs
+// (granule_offsets; a pair's last granule may be short).  Each warp takes runs
+// of granules from it and emits one granule at a time, converged.  What
+// follows differs by mode:
 //
 // Physical mode: photons end after very different numbers of steps (3.4 on
 // average in the mixed batch), so the warp stages emissions in a ring of
@@ -54,16 +57,17 @@ constexpr int kStage = 64;  // >= 2 * 32 - 1 staged emissions per warp (power of
 //   2: index lo, the first step's counter word, pair, the pair's sphere radius (a refill reads shared memory only)
 //   3: the step stream's words, a, q
 //
-// A warp's current photon chunk, with a copy of its pair's record, is kept in
-// shared memory too: only the emission pass reads or advances it, so the
-// step loop holds no registers for it.  A pass emits photons of one pair, so
-// it reads the record by broadcast.
+// The part of a warp's run that lies in one pair, with a copy of the pair's
+// record, is kept in shared memory too: only the emission pass reads or
+// advances it, so the step loop holds no registers for it.  A pass emits
+// photons of one pair, so it reads the record by broadcast.
 template <int MODE>
 struct __align__(16) WarpArea {
   float4 ring[4][MODE == kPhysical ? kStage : 1];
-  float4 rec[5];            // the chunk's pp_pair
-  unsigned long long base;  // next photon index of the chunk
-  unsigned left;            // photons left in the chunk
+  float4 rec[5];                       // the current pair's pp_pair
+  unsigned long long base;             // its next photon index
+  unsigned long long run_at, run_end;  // the granules of the run that follow in other pairs
+  unsigned left;                       // the pair's photons left in the run
   int pair;
   WarpStats stats;
 };
@@ -100,14 +104,15 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
     for (int k = 0; k < 6; ++k) wa->stats.v[k] = 0.0;
     wa->left = 0;
     wa->pair = 0;
+    wa->run_at = wa->run_end = 0;
   }
   __syncthreads();
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // what the set-up kernel writes is read below
 
   const unsigned lt_mask = (1u << lane) - 1u;
   WarpStats* ws = &wa->stats;
   StagedHit* hst = hstage[MODE == kCompat ? (threadIdx.x >> 5) : 0];
   unsigned h_count = 0;  // staged hits, warp-uniform
-  const unsigned long long total_chunks = R.chunk_offsets[R.n_pairs];
   // records staged hits 0..n-1 (n warp-uniform), one per lane
   auto record_staged = [&](unsigned n) {
     __syncwarp();
@@ -163,26 +168,40 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
       }
     }
   };
-  // the warp's next chunk of the queue, its pair's record and statistics
-  // cache; false when the queue is exhausted
+  // the next pair of the warp's run, or of its next run, with its record and
+  // statistics cache; false when the queue is exhausted.  A run is half the
+  // warps' share of what was left when the warp last looked, between one
+  // granule and R.max_run of them: long runs while there is much to do (a
+  // lookup per 4096 photons), short ones at the end, so that the warps finish
+  // together, and a small batch spreads over all of them.
   auto fetch = [&]() {
     int p = -1;
     if (lane == 0) {
-      const unsigned long long cid = atomicAdd(R.queue, 1ull);
-      if (cid < total_chunks) {
-        int hi = (int)R.n_pairs - 1;  // last pair whose first chunk <= cid
+      unsigned long long at = wa->run_at, end = wa->run_end;
+      const unsigned long long total = R.granule_offsets[R.n_pairs];
+      if (at >= end) {
+        const unsigned long long share = (total - min(end, total)) / (2u * gridDim.x * WARPS);
+        const unsigned long long n = max(1ull, min(share, (unsigned long long)R.max_run));
+        at = atomicAdd(R.queue, n);
+        end = min(at + n, total);
+      }
+      if (at < end) {
+        int hi = (int)R.n_pairs - 1;  // last pair whose first granule <= at
         p = 0;
         while (p < hi) {
           const int mid = (p + hi + 1) >> 1;
-          if (R.chunk_offsets[mid] <= cid) p = mid; else hi = mid - 1;
+          if (R.granule_offsets[mid] <= at) p = mid; else hi = mid - 1;
         }
-        const unsigned long long start = (cid - R.chunk_offsets[p]) * (unsigned long long)R.chunk;
+        const unsigned long long first = R.granule_offsets[p], stop = min(end, R.granule_offsets[p + 1]);
+        const unsigned long long start = (at - first) * 32u;
         wa->base = start;
-        wa->left = (unsigned)min((unsigned long long)R.chunk, (unsigned long long)R.pairs[p].n_photons - start);
+        wa->left = (unsigned)min((stop - at) * 32u, (unsigned long long)R.pairs[p].n_photons - start);
+        wa->run_at = stop;
+        wa->run_end = end;
         wa->pair = p;
         if (EM == kEmBasic && R.pairs[p].emitter == PP_EMITTER_CASCADE)
           atomicOr(R.counters + 2, 4ull);  // a cascade pair in a launch without PP_OPT_CASCADE
-        if (p != ws->pair) {               // the warp's statistics cache follows its chunk
+        if (p != ws->pair) {               // the warp's statistics cache follows its run
           flush_warp_stats(R.stats, ws);
           ws->pair = p;
         }
@@ -193,8 +212,8 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
     __syncwarp();
     return p >= 0;
   };
-  // emits the chunk's next photons, one per lane (lanes past its end emit as
-  // well, and drop it); returns whether the lane has one that is in reach
+  // emits the pair's next photons, one per lane (lanes past its last photon
+  // emit as well, and drop it); returns whether the lane has one that is in reach
   unsigned steps = 0;  // beyond the photons' first ones, which the set-up kernel has counted
   auto emit = [&](Photon& e, PairCtx& c) {
     const unsigned left = wa->left, n = min(32u, left);
@@ -413,85 +432,126 @@ __global__ void __launch_bounds__(1024) stacks_kernel(const RunParams R, const p
 }
 
 // ---------------------------------------------------------------------------
-// Chunk offsets of the work queue: offsets[p] = sum_{q<p} ceil(N_q / chunk),
-// offsets[n] = total.  One block; also resets the queue and counters.
-__global__ void __launch_bounds__(1024) chunk_scan_kernel(const pp_pair* __restrict__ pairs, int64_t n,
-                                                          uint32_t chunk,
-                                                          unsigned long long* __restrict__ offsets,
-                                                          unsigned long long* __restrict__ queue,
-                                                          unsigned long long* __restrict__ counters) {
-  __shared__ unsigned long long warp_sums[32];
-  const int t = threadIdx.x;
-  const int64_t per = (n + blockDim.x - 1) / blockDim.x;
-  const int64_t b = (int64_t)t * per;
-  const int64_t e = min(b + per, n);
-  unsigned long long local = 0;
-  for (int64_t i = b; i < e; ++i) {
-    const long long np = pairs[i].n_photons;
-    local += np > 0 ? ((unsigned long long)np + chunk - 1) / chunk : 0ull;
-  }
-  // exclusive block scan of `local`
-  const unsigned lane = t & 31, warp = t >> 5;
-  unsigned long long incl = local;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long v = __shfl_up_sync(kFull, incl, o);
-    if ((int)lane >= o) incl += v;
-  }
-  if (lane == 31) warp_sums[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    unsigned long long w = (lane < (blockDim.x >> 5)) ? warp_sums[lane] : 0ull;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long v = __shfl_up_sync(kFull, w, o);
-      if ((int)lane >= o) w += v;
+// The outputs of a launch before it: statistics rows (zeros, and the photon
+// count in column 6) and zeroed histograms, by threads first, first + stride, ...
+__device__ __forceinline__ void fill_outputs(const pp_pair* __restrict__ pairs, int64_t n, double* __restrict__ stats,
+                                             double* __restrict__ hist, int64_t hist_len, int64_t first,
+                                             int64_t stride) {
+  if (stats)
+    for (int64_t i = first; i < n * PP_STATS; i += stride)
+      stats[i] = i % PP_STATS == 6 ? (double)pairs[i / PP_STATS].n_photons : 0.0;
+  if (hist) {  // 16-byte stores from the first 16-byte boundary on
+    const int64_t head = min((int64_t)((reinterpret_cast<uintptr_t>(hist) >> 3) & 1u), hist_len);
+    double2* body = reinterpret_cast<double2*>(hist + head);
+    const int64_t nb = (hist_len - head) / 2;
+    for (int64_t i = first; i < nb; i += stride) body[i] = make_double2(0.0, 0.0);
+    if (first == 0) {
+      if (head) hist[0] = 0.0;
+      if (head + 2 * nb < hist_len) hist[hist_len - 1] = 0.0;
     }
-    warp_sums[lane] = w;  // inclusive over warps
   }
+}
+
+__global__ void __launch_bounds__(1024) fill_kernel(const pp_pair* __restrict__ pairs, int64_t n,
+                                                    double* __restrict__ stats, double* __restrict__ hist,
+                                                    int64_t hist_len) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // setup_kernel scans meanwhile
+  fill_outputs(pairs, n, stats, hist, hist_len, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
+               (int64_t)gridDim.x * blockDim.x);
+}
+
+// The work queue of a launch.  Block 0 resets the queue cursor and the
+// counters and writes the offsets: offsets[p] = granules (32 photons) of pairs
+// 0..p-1, offsets[n] all of them; counters[1] starts as the photons' first
+// steps (one each), to which the batched kernel adds the others.  offsets ==
+// NULL (the one-pair kernel, which counts all its steps): no queue.  Further
+// blocks, if any, fill the outputs.
+__global__ void __launch_bounds__(1024) setup_kernel(const pp_pair* __restrict__ pairs, int64_t n,
+                                                     unsigned long long* __restrict__ offsets,
+                                                     unsigned long long* __restrict__ queue,
+                                                     unsigned long long* __restrict__ counters,
+                                                     double* __restrict__ stats, double* __restrict__ hist,
+                                                     int64_t hist_len) {
+  // the batched kernel may start (its blocks wait for this grid to end
+  // before they read what it writes)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int t = threadIdx.x;
+  if (blockIdx.x > 0) {
+    fill_outputs(pairs, n, stats, hist, hist_len, (int64_t)(blockIdx.x - 1) * blockDim.x + t,
+                 (int64_t)(gridDim.x - 1) * blockDim.x);
+    return;
+  }
+  __shared__ unsigned long long granules[32], photons[32];
+  const unsigned lane = t & 31, warp = t >> 5;
+  unsigned long long done = 0, seen = 0;  // granules of the tiles before; this thread's photons
+  constexpr int kPer = 4;                 // pairs per thread and tile, loaded together
+  if (offsets) {
+    for (int64_t tile = 0; tile < n; tile += (int64_t)kPer * blockDim.x) {
+      unsigned long long g[kPer], sum = 0;
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) {
+        const int64_t i = tile + (int64_t)t * kPer + j;
+        const long long np = i < n ? (long long)__ldg(reinterpret_cast<const long long*>(pairs + i) + 6) : 0ll;
+        g[j] = np > 0 ? (unsigned long long)np : 0ull;
+      }
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) {
+        seen += g[j];
+        g[j] = (g[j] + 31u) / 32u;
+        sum += g[j];
+      }
+      unsigned long long incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long v = __shfl_up_sync(kFull, incl, o);
+        if ((int)lane >= o) incl += v;
+      }
+      if (lane == 31) granules[warp] = incl;
+      __syncthreads();
+      unsigned long long before = done, all = 0;
+#pragma unroll
+      for (unsigned w = 0; w < 32; ++w) {  // 32 warps: read by broadcast
+        before += w < warp ? granules[w] : 0ull;
+        all += granules[w];
+      }
+      __syncthreads();
+      unsigned long long run = before + incl - sum;
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) {
+        const int64_t i = tile + (int64_t)t * kPer + j;
+        if (i < n) offsets[i] = run;
+        run += g[j];
+      }
+      done += all;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) seen += __shfl_xor_sync(kFull, seen, o);
+  if (lane == 0) photons[warp] = seen;
   __syncthreads();
-  unsigned long long run = incl - local + (warp > 0 ? warp_sums[warp - 1] : 0ull);
-  for (int64_t i = b; i < e; ++i) {
-    offsets[i] = run;
-    const long long np = pairs[i].n_photons;
-    run += np > 0 ? ((unsigned long long)np + chunk - 1) / chunk : 0ull;
-  }
-  if (t == (int)blockDim.x - 1) offsets[n] = warp_sums[(blockDim.x >> 5) - 1];
   if (t == 0) {
-    queue[0] = 0ull;
+    unsigned long long all = 0;
+    for (int w = 0; w < 32; ++w) all += photons[w];
+    if (offsets) {
+      offsets[n] = done;
+      queue[0] = 0ull;
+    }
     counters[0] = 0ull;
+    counters[1] = all;
     counters[2] = 0ull;
     counters[3] = 0ull;
   }
-  // counters[1] starts as the photons' first steps; the batched kernel adds the others
-  unsigned long long photons = 0;
-  for (int64_t i = b; i < e; ++i) photons += (unsigned long long)max((long long)pairs[i].n_photons, 0ll);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) photons += __shfl_xor_sync(kFull, photons, o);
-  __syncthreads();
-  if (lane == 0) warp_sums[warp] = photons;
-  __syncthreads();
-  if (t == 0) {
-    unsigned long long sum = 0;
-    for (unsigned w = 0; w < (blockDim.x >> 5); ++w) sum += warp_sums[w];
-    counters[1] = sum;
-  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // fill_kernel, where it ran before: its end is part of this grid's
 }
 
-__global__ void reset_counters_kernel(unsigned long long* __restrict__ counters) {
-  if (threadIdx.x < 4) counters[threadIdx.x] = 0ull;
-}
-
-// stats[p][6] = photons; optionally hist[p][:] /= photons.
-__global__ void finalize_kernel(const pp_pair* __restrict__ pairs, int64_t n_pairs, double* __restrict__ stats,
-                                double* __restrict__ hist, int bins, int normalize) {
-  const int64_t total = n_pairs * (int64_t)(bins > 0 ? bins : 1);
+// hist[p][:] /= photons.
+__global__ void normalize_kernel(const pp_pair* __restrict__ pairs, int64_t n_pairs, double* __restrict__ hist,
+                                 int bins) {
+  const int64_t total = n_pairs * (int64_t)bins;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = bins > 0 ? i / bins : i;
-    const double n = (double)pairs[p].n_photons;
-    if (bins <= 0 || i % bins == 0) stats[p * PP_STATS + 6] = n;
-    if (normalize && bins > 0 && n > 0) hist[i] /= n;
+    const double n = (double)pairs[i / bins].n_photons;
+    if (n > 0) hist[i] /= n;
   }
 }
 
@@ -648,9 +708,9 @@ static __host__ ppd::RunParams to_params(const LaunchArgs& a) {
   ppd::RunParams R;
   R.pairs = a.pairs;
   R.n_pairs = a.n_pairs;
-  R.chunk_offsets = a.chunk_offsets;
+  R.granule_offsets = a.granule_offsets;
   R.queue = a.queue;
-  R.chunk = a.chunk;
+  R.max_run = std::max(1u, a.chunk / 32u + (a.chunk % 32u != 0u));
   R.pair_base = a.pair_base;
   R.hits = a.hits;
   R.hit_cap = a.hit_cap;
@@ -720,38 +780,68 @@ void get_dev_knots(const void* host_tables, float* out, int* n) {
   for (int i = 0; i < t->n_knots; ++i) out[i] = t->knots[i];
 }
 
-cudaError_t launch_chunk_scan(const LaunchArgs& a, cudaStream_t s) {
-  ppd::chunk_scan_kernel<<<1, 1024, 0, s>>>(a.pairs, a.n_pairs, a.chunk, a.chunk_offsets, a.queue, a.counters);
+// A launch that may start while the kernel before it on the stream runs (its
+// programmatic dependent): it waits itself, by griddepcontrol.wait, before it
+// reads what that kernel writes.
+template <typename... P, typename... A>
+static cudaError_t launch_dependent(void (*fn)(P...), int grid, int block, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, P(args)...);
   count_launches(1);
-  return cudaGetLastError();
+  return e;
 }
 
-cudaError_t launch_reset_counters(unsigned long long* counters, cudaStream_t s) {
-  ppd::reset_counters_kernel<<<1, 32, 0, s>>>(counters);
+cudaError_t launch_setup(const LaunchArgs& a, int sm_count, cudaStream_t s) {
+  const int64_t hist_len = a.hist ? a.n_pairs * (int64_t)a.opts.hist_bins : 0;
+  const int64_t words = (a.stats ? a.n_pairs * PP_STATS : 0) + hist_len;
+  // 16 words per thread.  What one block fills (a single source, 16 pairs of
+  // 1000 bins) is a second block of the set-up kernel, one launch less; beyond,
+  // the outputs have a kernel of their own, which the scan's registers do not
+  // hold to one block per SM.
+  const int64_t blocks = (words + 16383) / 16384;
+  if (blocks <= 1) {
+    ppd::setup_kernel<<<1 + (int)blocks, 1024, 0, s>>>(a.pairs, a.n_pairs, a.granule_offsets, a.queue, a.counters,
+                                                       a.stats, a.hist, hist_len);
+    count_launches(1);
+    return cudaGetLastError();
+  }
+  ppd::fill_kernel<<<(int)std::min<int64_t>(blocks, 2 * (int64_t)sm_count), 1024, 0, s>>>(a.pairs, a.n_pairs, a.stats,
+                                                                                          a.hist, hist_len);
   count_launches(1);
-  return cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
+  if (e) return e;
+  return launch_dependent(ppd::setup_kernel, 1, 1024, s, a.pairs, a.n_pairs, a.granule_offsets, a.queue, a.counters,
+                          (double*)nullptr, (double*)nullptr, (int64_t)0);
 }
 
+namespace {
+using BatchedFn = void (*)(ppd::RunParams);
+BatchedFn batched_fn(int mode, int block, bool cascade) {
+  if (mode == PP_MODE_COMPAT)
+    return block == 128 ? ppd::batched_kernel<ppd::kCompat, 4, ppd::kEmBasic>
+                        : ppd::batched_kernel<ppd::kCompat, 8, ppd::kEmBasic>;
+  if (cascade)
+    return block == 128 ? ppd::batched_kernel<ppd::kPhysical, 4, ppd::kEmCascade>
+                        : ppd::batched_kernel<ppd::kPhysical, 8, ppd::kEmCascade>;
+  return block == 128 ? ppd::batched_kernel<ppd::kPhysical, 4, ppd::kEmBasic>
+                      : ppd::batched_kernel<ppd::kPhysical, 8, ppd::kEmBasic>;
+}
+}  // namespace
+
+// Follows launch_setup on the same stream: the blocks start and stage their
+// tables while the set-up kernel runs, then wait for it to end.
 cudaError_t launch_batched(const LaunchArgs& a, int grid, int block, cudaStream_t s) {
   const ppd::RunParams R = to_params(a);
-  const bool casc = a.opts.mode == PP_MODE_PHYSICAL && (a.opts.flags & PP_OPT_CASCADE);
-  if (block == 128) {
-    if (a.opts.mode == PP_MODE_COMPAT)
-      ppd::batched_kernel<ppd::kCompat, 4, ppd::kEmBasic><<<grid, 128, 0, s>>>(R);
-    else if (casc)
-      ppd::batched_kernel<ppd::kPhysical, 4, ppd::kEmCascade><<<grid, 128, 0, s>>>(R);
-    else
-      ppd::batched_kernel<ppd::kPhysical, 4, ppd::kEmBasic><<<grid, 128, 0, s>>>(R);
-  } else {
-    if (a.opts.mode == PP_MODE_COMPAT)
-      ppd::batched_kernel<ppd::kCompat, 8, ppd::kEmBasic><<<grid, 256, 0, s>>>(R);
-    else if (casc)
-      ppd::batched_kernel<ppd::kPhysical, 8, ppd::kEmCascade><<<grid, 256, 0, s>>>(R);
-    else
-      ppd::batched_kernel<ppd::kPhysical, 8, ppd::kEmBasic><<<grid, 256, 0, s>>>(R);
-  }
-  count_launches(1);
-  return cudaGetLastError();
+  if (block != 128) block = 256;
+  return launch_dependent(batched_fn(a.opts.mode, block, (a.opts.flags & PP_OPT_CASCADE) != 0), grid, block, s, R);
 }
 
 cudaError_t launch_plain(const LaunchArgs& a, const pp_pair* d_pair, int pair_index, int grid, int block,
@@ -783,12 +873,10 @@ cudaError_t launch_stacks(const LaunchArgs& a, const pp_pair* d_pair, float* pos
   return cudaGetLastError();
 }
 
-cudaError_t launch_finalize(const pp_pair* pairs, int64_t n, double* stats, double* hist, int bins, int normalize,
-                            int sm_count, cudaStream_t s) {
-  const int64_t total = n * (int64_t)(bins > 0 ? bins : 1);
-  int grid = (int)std::min<int64_t>((total + 255) / 256, (int64_t)sm_count * 8);
-  if (grid < 1) grid = 1;
-  ppd::finalize_kernel<<<grid, 256, 0, s>>>(pairs, n, stats, hist, bins, normalize);
+cudaError_t launch_normalize(const pp_pair* pairs, int64_t n, double* hist, int bins, int sm_count, cudaStream_t s) {
+  const int64_t total = n * (int64_t)bins;
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, (int64_t)sm_count * 8));
+  ppd::normalize_kernel<<<grid, 256, 0, s>>>(pairs, n, hist, bins);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -802,22 +890,8 @@ cudaError_t launch_eval(int op, const double* in, double* out, int64_t n, const 
 
 int batched_max_blocks_per_sm(int mode, int block, bool cascade) {
   int nb = 0;
-  const bool c = mode == PP_MODE_PHYSICAL && cascade;
-  if (block == 128) {
-    if (mode == PP_MODE_COMPAT)
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ppd::batched_kernel<ppd::kCompat, 4, ppd::kEmBasic>, 128, 0);
-    else if (c)
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ppd::batched_kernel<ppd::kPhysical, 4, ppd::kEmCascade>, 128, 0);
-    else
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ppd::batched_kernel<ppd::kPhysical, 4, ppd::kEmBasic>, 128, 0);
-  } else {
-    if (mode == PP_MODE_COMPAT)
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ppd::batched_kernel<ppd::kCompat, 8, ppd::kEmBasic>, 256, 0);
-    else if (c)
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ppd::batched_kernel<ppd::kPhysical, 8, ppd::kEmCascade>, 256, 0);
-    else
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ppd::batched_kernel<ppd::kPhysical, 8, ppd::kEmBasic>, 256, 0);
-  }
+  if (block != 128) block = 256;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batched_fn(mode, block, cascade), block, 0);
   return nb;
 }
 

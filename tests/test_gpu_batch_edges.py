@@ -76,3 +76,46 @@ def test_step_count_of_photons_out_of_reach(propagator):
     propagator.propagate_device(d_pairs, 3, ro, hits, 0, cnt, st, None)
     torch.cuda.synchronize()
     assert cnt.tolist() == [0, int(pairs["n_photons"].sum()), 0, 0]
+
+
+@pytest.mark.parametrize("n_pairs,chunk", [(1, 0), (3, 1), (4095, 33), (4096, 0), (4097, 100_000), (9001, 0)])
+def test_work_queue_covers_every_photon(propagator, n_pairs, chunk):
+    """Tiles of the set-up scan (4096 pairs), empty pairs and run lengths: every photon is propagated exactly once
+    (the same hits and step count as one launch per pair, histograms that start 8 bytes off a 16-byte boundary)."""
+    import torch
+    dev = torch.device("cuda:0")
+    rng = np.random.default_rng(n_pairs)
+    counts = rng.integers(0, 200, n_pairs) * (rng.uniform(size=n_pairs) < 0.7)
+    counts[rng.integers(0, n_pairs)] = 100_000
+    pairs = _pairs(counts, np.full(n_pairs, 1.2), False, n_pairs)
+    bins, cap = 31, 1 << 16
+    ro = pp.RunOptions(mode="physical", t_max=31.0, hist_bins=bins, chunk_photons=chunk)
+    d_pairs = torch.from_numpy(pairs.view(np.uint8).copy()).to(dev)
+    hits = torch.zeros(cap * 64, dtype=torch.uint8, device=dev)
+    cnt = torch.full((4,), 7, dtype=torch.int64, device=dev)
+    st = torch.full((n_pairs, 8), 3.0, dtype=torch.float64, device=dev)
+    flat = torch.full((n_pairs * bins + 2,), 5.0, dtype=torch.float64, device=dev)
+    propagator.propagate_device(d_pairs, n_pairs, ro, hits, cap, cnt, st, flat[1:-1])
+    torch.cuda.synchronize()
+    n = int(cnt[0])
+    h = hits[:n * 64].cpu().numpy().view(pp.HIT_DTYPE)
+    h = h[np.lexsort((h["photon"], h["pair"]))]
+    want = propagator.propagate_plain(pairs[counts > 0], ro, hit_capacity=cap)
+    w = want.sorted_hits()
+    w["pair"] = np.flatnonzero(counts > 0)[w["pair"]]
+    np.testing.assert_array_equal(h.view(np.uint8), w.view(np.uint8))
+    steps = 0  # photons are a function of (seed, index): a pair alone makes the same steps
+    one_cnt = torch.zeros(4, dtype=torch.int64, device=dev)
+    for i in rng.permutation(np.flatnonzero(counts > 0))[:20] if n_pairs > 20 else np.flatnonzero(counts > 0):
+        propagator.propagate_plain_device(d_pairs[80 * i:], pairs[i:i + 1], 0, ro, hits, 0, one_cnt, st[i:i + 1],
+                                          torch.zeros(bins, dtype=torch.float64, device=dev))
+        steps += int(one_cnt[1])
+    if n_pairs <= 20:
+        assert steps == int(cnt[1])
+    assert int(cnt[1]) >= int(counts.sum()) and cnt[2:].tolist() == [1 if n > cap else 0, 0]
+    s = st.cpu().numpy()
+    np.testing.assert_array_equal(s[:, 6], counts)
+    np.testing.assert_array_equal(np.bincount(h["pair"], minlength=n_pairs), s[:, 0])
+    assert float(flat[0]) == 5.0 and float(flat[-1]) == 5.0
+    hist = flat[1:-1].reshape(n_pairs, bins).cpu().numpy()
+    np.testing.assert_allclose(hist.sum(1), s[:, 1], rtol=1e-12, atol=1e-300)
