@@ -42,6 +42,26 @@ struct LaunchArgs {
 
 void count_launches(uint64_t n);
 
+// A launch that may start while the kernel before it on the stream runs (its
+// programmatic dependent): it waits itself, by griddepcontrol.wait, before it
+// reads what that kernel writes.
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*fn)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, P(args)...);
+  count_launches(1);
+  return e;
+}
+
 size_t dev_tables_size();
 // coeffs: a01, a2, a3, a4, sca0, sca1, sca2 (+ unused)
 void fill_dev_tables(void* host_tables, const double coeffs[11], const float* knots, int n_knots,

@@ -780,25 +780,6 @@ void get_dev_knots(const void* host_tables, float* out, int* n) {
   for (int i = 0; i < t->n_knots; ++i) out[i] = t->knots[i];
 }
 
-// A launch that may start while the kernel before it on the stream runs (its
-// programmatic dependent): it waits itself, by griddepcontrol.wait, before it
-// reads what that kernel writes.
-template <typename... P, typename... A>
-static cudaError_t launch_dependent(void (*fn)(P...), int grid, int block, cudaStream_t s, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)block);
-  cfg.stream = s;
-  cudaLaunchAttribute at = {};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, P(args)...);
-  count_launches(1);
-  return e;
-}
-
 cudaError_t launch_setup(const LaunchArgs& a, int sm_count, cudaStream_t s) {
   const int64_t hist_len = a.hist ? a.n_pairs * (int64_t)a.opts.hist_bins : 0;
   const int64_t words = (a.stats ? a.n_pairs * PP_STATS : 0) + hist_len;
@@ -818,7 +799,7 @@ cudaError_t launch_setup(const LaunchArgs& a, int sm_count, cudaStream_t s) {
   count_launches(1);
   const cudaError_t e = cudaGetLastError();
   if (e) return e;
-  return launch_dependent(ppd::setup_kernel, 1, 1024, s, a.pairs, a.n_pairs, a.granule_offsets, a.queue, a.counters,
+  return launch_dependent(ppd::setup_kernel, 1, 1024, 0, s, a.pairs, a.n_pairs, a.granule_offsets, a.queue, a.counters,
                           (double*)nullptr, (double*)nullptr, (int64_t)0);
 }
 
@@ -841,7 +822,7 @@ BatchedFn batched_fn(int mode, int block, bool cascade) {
 cudaError_t launch_batched(const LaunchArgs& a, int grid, int block, cudaStream_t s) {
   const ppd::RunParams R = to_params(a);
   if (block != 128) block = 256;
-  return launch_dependent(batched_fn(a.opts.mode, block, (a.opts.flags & PP_OPT_CASCADE) != 0), grid, block, s, R);
+  return launch_dependent(batched_fn(a.opts.mode, block, (a.opts.flags & PP_OPT_CASCADE) != 0), grid, block, 0, s, R);
 }
 
 cudaError_t launch_plain(const LaunchArgs& a, const pp_pair* d_pair, int pair_index, int grid, int block,

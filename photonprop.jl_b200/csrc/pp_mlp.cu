@@ -1,24 +1,19 @@
 // Learned surrogate: MLP 4 -> 128 -> 128 -> 128 -> 5 with GELU, on sm_100a.
 //
-// Every CTA owns a tile of 128 rows (queries), one row per thread (4 warps).
+// A tile is 128 rows (queries).
 // The 128 x 128 layers run on the 5th-generation tensor cores: one thread
 // issues eight tcgen05.mma (M = N = 128, K = 16, BF16 inputs, FP32
 // accumulation in tensor memory) per layer, commits them to an mbarrier, and
 // every warp reads its 32 rows back with tcgen05.ld; bias, GELU and the BF16
-// conversion of the next layer's operand are fused into that read-back.  The
-// 4-wide input layer and the 5-wide output layer are too narrow for the tensor
-// cores and run on the FP32 pipes with BF16-rounded weights.
+// conversion of the next layer's operand are fused into that read-back.
 //
 // Operand tiles live in shared memory in the no-swizzle K-major canonical
 // layout: 8-row x 16-byte core matrices, core matrices along K 128 bytes apart
 // (leading byte offset), 8-row groups 2048 bytes apart (stride byte offset).
 //
-// Training (one fused kernel per 128-row tile): forward with the activations
-// saved, masked-MSE loss, backward through all layers; the weight gradients of
-// the 128 x 128 layers are tcgen05 GEMMs over the tile's rows (the transposed
-// operands are written transposed into shared memory) accumulated across tiles
-// with FP32 atomics; then an Adam kernel updates the FP32 master weights and
-// rebuilds the BF16 tensor-core copies.
+// Training: one fused kernel per 128-row tile (forward, masked-MSE loss and
+// backward, see train_kernel), then an Adam kernel that updates the FP32
+// master weights and their BF16 tensor-core copies.
 //
 // Every mbarrier wait is bounded (iteration and clock limits); on expiry the
 // kernel sets an error flag, stops issuing work and frees its tensor memory.
@@ -49,9 +44,13 @@ __host__ __device__ __forceinline__ int tc_offset(int row, int k) {
   return (((row >> 3) * 16 + (k >> 3)) << 6) + ((row & 7) << 3) + (k & 7);
 }
 
-__device__ __forceinline__ float gelu(float z) {
+// Training's GELU and its derivative, from one (accurate) tanh.
+__device__ __forceinline__ void gelu_both(float z, float& h, float& g) {
   const float u = 0.7978845608028654f * fmaf(0.044715f * z, z * z, z);
-  return 0.5f * z * (1.f + tanhf(u));
+  const float t = tanhf(u);
+  h = 0.5f * z * (1.f + t);
+  const float du = 0.7978845608028654f * fmaf(3.f * 0.044715f, z * z, 1.f);
+  g = 0.5f * (1.f + t) + 0.5f * z * (1.f - t * t) * du;
 }
 // Twice the inference GELU with the MUFU tanh (tanh.approx.f32, relative
 // error below 2^-10, under the BF16 rounding that follows it), in four FP32
@@ -75,12 +74,6 @@ __device__ __forceinline__ float2 gelu2_fast2(float2 z) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(t.x) : "f"(u.x));
   asm("tanh.approx.f32 %0, %1;" : "=f"(t.y) : "f"(u.y));
   return __ffma2_rn(z, t, z);
-}
-__device__ __forceinline__ float gelu_grad(float z) {
-  const float u = 0.7978845608028654f * fmaf(0.044715f * z, z * z, z);
-  const float t = tanhf(u);
-  const float du = 0.7978845608028654f * fmaf(3.f * 0.044715f, z * z, 1.f);
-  return 0.5f * (1.f + t) + 0.5f * z * (1.f - t * t) * du;
 }
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
@@ -222,16 +215,12 @@ __device__ __forceinline__ uint32_t lane_taddr(uint32_t tmem) { return tmem + ((
 // Device parameter block.
 struct DevParams {
   const float* p;        // FP32 master parameters (N_PARAMS)
-  const float* w1r;      // BF16-rounded W1 [128][4]
-  const float* w4r;      // BF16-rounded W4 [5][128]
-  const __nv_bfloat16* w2tc;   // W2 as the B operand of h W2^T (canonical tile)
-  const __nv_bfloat16* w3tc;
-  const __nv_bfloat16* w1tc;   // W1 as the B operand of x W1^T: 128 rows x K 16 (4 used)
-  const __nv_bfloat16* w4tc;   // W4 / 2 as the B operand of h W4^T: 16 rows (5 used) x K 128
-  const __nv_bfloat16* w2h;    // W2 / 2, W3 / 2: inference B operands (they take 2 GELU)
+  const __nv_bfloat16* w2tc;  // W2, W3 as canonical tiles (rows = out, columns = in): the B operand of
+  const __nv_bfloat16* w3tc;  // h W^T read K-major, and of dz W read MN-major
+  const __nv_bfloat16* w2h;   // W2 / 2, W3 / 2: inference B operands (they take 2 GELU)
   const __nv_bfloat16* w3h;
-  const __nv_bfloat16* w2ttc;  // W2^T as the B operand of dz W2
-  const __nv_bfloat16* w3ttc;
+  const __nv_bfloat16* w1tc;  // W1 as the B operand of x W1^T: 128 rows x K 16 (4 used, then b1 in two)
+  const __nv_bfloat16* w4tc;  // W4 / 2 as the B operand of h W4^T: 16 rows (5 used) x K 128
   const float* norm;     // x_mean[4], x_std[4], y_mean[5], y_std[5]
   int* error;
 };
@@ -467,275 +456,444 @@ __global__ void __launch_bounds__(INFER_THREADS, 1) infer_kernel(DevParams P, co
 }
 
 // ---------------------------------------------------------------------------
-// Training, one CTA per 128-row tile.  xn [n][4] standardised features,
-// yt [n][5] standardised targets, mask [n][5]; grads (N_PARAMS) accumulated
-// with atomics; loss_sum += sum of mask * (y - t)^2; inv_count = 1 / sum(mask).
-// Scratch: z [3][n][128] FP32 pre-activations, h [3][n][128] BF16 activations.
-__global__ void __launch_bounds__(THREADS, 1) train_kernel(DevParams P, const float* __restrict__ xn,
-                                                          const float* __restrict__ yt,
-                                                          const float* __restrict__ mask, int64_t n,
-                                                          float inv_count, float* __restrict__ grad,
-                                                          float* __restrict__ loss_sum, float* __restrict__ zs,
-                                                          __nv_bfloat16* __restrict__ hs) {
+// Training.  count_kernel zeroes the gradients and the loss and sums the mask
+// in FP64 (kCountBlocks partial sums, added in one order by every reader);
+// train_kernel adds a tile's gradients; adam_kernel applies them.
+constexpr int kCountBlocks = 32;
+// What a step brings back: the gradients, the loss sum, the error flag, the mask sums (doubles).
+constexpr int kPartAt = (N_PARAMS + 3) & ~1, kBack = kPartAt + 2 * kCountBlocks;
+
+__global__ void __launch_bounds__(256) count_kernel(const float* __restrict__ mask, int64_t count,
+                                                    float* __restrict__ grad, double* __restrict__ part) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = first; i < N_PARAMS + 1; i += stride) grad[i] = 0.f;  // and the loss
+  double s = 0.0;
+  for (int64_t i = first; i < count; i += stride) s += (double)mask[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  __shared__ double warp[8];
+  if ((threadIdx.x & 31u) == 0) warp[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) t += warp[w];
+    part[blockIdx.x] = t;
+  }
+}
+
+// FP32 columns [0, 32) to this thread's row of tensor memory.
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+      "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]),
+      "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]), "f"(v[16]), "f"(v[17]), "f"(v[18]),
+      "f"(v[19]), "f"(v[20]), "f"(v[21]), "f"(v[22]), "f"(v[23]), "f"(v[24]), "f"(v[25]), "f"(v[26]), "f"(v[27]),
+      "f"(v[28]), "f"(v[29]), "f"(v[30]), "f"(v[31]));
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// Sums of 32 values over the 32 lanes of a warp: lane l returns the sum of
+// v[l] (31 shuffles: each halving step keeps one half of the values and adds
+// the partner's).
+__device__ __forceinline__ float warp_column_sum(float* v) {
+  const unsigned lane = threadIdx.x & 31u;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool upper = lane & o;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const float keep = upper ? v[i + o] : v[i], give = upper ? v[i] : v[i + o];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  return v[0];
+}
+
+// Adds a 512-byte row of FP32 in shared memory to global memory.
+__device__ __forceinline__ void bulk_add_row(float* dst, const void* src) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], 512;" ::"l"(dst),
+               "r"(smem_u32(src))
+               : "memory");
+}
+
+// A and B both MN-major (bits 15 and 16), or B alone.
+constexpr uint32_t kIdescMnMn = kIdesc | (1u << 15) | (1u << 16), kIdescKMn = kIdesc | (1u << 16);
+
+// One CTA of 512 threads per 128-row tile.  xn [n][4] standardised features,
+// yt [n][5] standardised targets, mask [n][5]; grad (N_PARAMS, then the loss
+// sum) accumulated with atomics; loss += sum of mask * (y - t)^2.
+//
+// Warp w holds the tile's rows 32 (w mod 4) .. + 31 (its tensor-memory lanes),
+// one per lane, and columns 32 (w / 4) .. + 31 of every layer.  Nothing goes
+// through global memory between layers: the activations h1, h2 stay in shared
+// memory as BF16 operand tiles, and the GELU derivatives of all three layers,
+// computed in the forward pass from the same tanh, in tensor memory (three
+// quarters of it; the fourth holds weight gradients, and a layer's quarter
+// takes its dh once its derivative is read).  An operand tile has 8 x 8 core
+// matrices, so one tile serves as a K-major operand in the forward pass and
+// MN-major in the backward pass (dW = dz^T h, dh = dz W): nothing is
+// transposed.  Bias gradients are warp column sums, the weight gradients go
+// from tensor memory through padded shared rows to global memory as bulk
+// additions of 512 bytes.
+//
+// What bounds it: three dependent layers forward and three back on one SM,
+// with 96 accurate tanh per thread (4096 rows are 32 CTAs).  Before, one warp
+// per 32 rows walked 128 columns with all activations in global memory and
+// every thread adding its bias gradients to the same addresses: 950-1080 us
+// for 4096 rows (32 tiles), now 36 us.
+constexpr int TRAIN_THREADS = 512;
+constexpr int kGradPitch = 528;  // bytes of a staged gradient row: 16-byte lanes of 8 rows fall on different banks
+
+__global__ void __launch_bounds__(TRAIN_THREADS, 1) train_kernel(DevParams P, const float* __restrict__ xn,
+                                                                const float* __restrict__ yt,
+                                                                const float* __restrict__ mask, int64_t n,
+                                                                const double* __restrict__ part,
+                                                                float* __restrict__ grad) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  __nv_bfloat16* ta = reinterpret_cast<__nv_bfloat16*>(smem_raw);  // A operand
-  __nv_bfloat16* tb = ta + TILE * H;                                 // B operand
-  __nv_bfloat16* tt = tb + TILE * H;                                 // transposed gradient (A of dW)
-  float* w1 = reinterpret_cast<float*>(tt + TILE * H);
-  float* w4 = w1 + H * IN;
-  float* b4 = w4 + OUT * H;
-  float* dys = b4 + 8;            // [128][5]
-  float* red = dys + TILE * OUT;  // [4] loss partials
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(red + 8);
+  // W2 H1 W3 H2 DZ3 DZ2, 32 KB each; reused as they fall free:
+  unsigned char* const base = smem_raw;
+  __nv_bfloat16* w2 = reinterpret_cast<__nv_bfloat16*>(base);
+  __nv_bfloat16* h1 = reinterpret_cast<__nv_bfloat16*>(base + TILE_BYTES);
+  __nv_bfloat16* w3 = reinterpret_cast<__nv_bfloat16*>(base + 2 * TILE_BYTES);
+  __nv_bfloat16* h2 = reinterpret_cast<__nv_bfloat16*>(base + 3 * TILE_BYTES);
+  __nv_bfloat16* dz3 = reinterpret_cast<__nv_bfloat16*>(base + 4 * TILE_BYTES);
+  __nv_bfloat16* dz2 = reinterpret_cast<__nv_bfloat16*>(base + 5 * TILE_BYTES);
+  unsigned char* const h3s = base + 5 * TILE_BYTES;         // h3, BF16 rows, until dz2
+  unsigned char* const gw3 = base + 2 * TILE_BYTES + 2048;  // dW3 rows, once w3, h2 and dz3 are free
+  unsigned char* const gw2 = base;                          // dW2 rows, once w2 and h1 are free (to 2 KB into w3)
+  unsigned char* const dz1s = base + 4 * TILE_BYTES;        // dz1, FP32 rows, once dz3 and dz2 are free: 64 KB
+  static_assert(2048 + TILE * kGradPitch <= 3 * TILE_BYTES && TILE * kGradPitch <= 2 * TILE_BYTES + 2048,
+                "staged gradients fit the tiles they replace");
+  float* w1 = reinterpret_cast<float*>(base + 6 * TILE_BYTES);  // [128][4]
+  float* w4 = w1 + H * IN;                                      // [128][8], 5 used
+  float* dys = w4 + H * 8;                                      // [128][8], 5 used
+  float* xs = dys + TILE * 8;                                   // [128][4], BF16-rounded
+  float* b123 = xs + TILE * IN;                                 // [3][128]
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(b123 + 3 * H);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 1);
 
-  const int t = threadIdx.x;
-  const int64_t row = (int64_t)blockIdx.x * TILE + t;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int r = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 32;  // this thread's row and first column
+  const int64_t row = (int64_t)blockIdx.x * TILE + r;
   const bool valid = row < n;
-  for (int i = t; i < H * IN; i += THREADS) w1[i] = P.w1r[i];
-  for (int i = t; i < OUT * H; i += THREADS) w4[i] = P.w4r[i];
-  if (t < OUT) b4[t] = P.p[OFF_B4 + t];
+  load_tile(w2, P.w2tc);
+  load_tile(w3, P.w3tc);
+  for (int i = t; i < H * IN; i += TRAIN_THREADS) w1[i] = bf16r(P.p[OFF_W1 + i]);
+  for (int i = t; i < OUT * H; i += TRAIN_THREADS) w4[(i % H) * 8 + i / H] = bf16r(P.p[OFF_W4 + i]);
+  if (t < H) {
+    b123[t] = P.p[OFF_B1 + t];
+    b123[H + t] = P.p[OFF_B2 + t];
+    b123[2 * H + t] = P.p[OFF_B3 + t];
+  }
+  float x[IN];
+#pragma unroll
+  for (int j = 0; j < IN; ++j) x[j] = valid ? bf16r(xn[row * IN + j]) : 0.f;
+  if (c0 == 0) *reinterpret_cast<float4*>(xs + r * IN) = make_float4(x[0], x[1], x[2], x[3]);
   if (t == 0) mbar_init(smem_u32(mbar));
-  tmem_alloc(tslot);
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tslot)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tslot;
+  const uint32_t tm = *tslot;  // g1 [0, 128), g2 / dh1 [128, 256), g3 / dh2 [256, 384), dW [384, 512)
+  const uint32_t ta = tm + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;  // this thread's lanes and columns
   const uint32_t mb = smem_u32(mbar);
   uint32_t parity = 0;
   bool ok = true;
-  const int64_t rr = valid ? row : 0;  // scratch row (invalid rows compute on zeros, contribute nothing)
-  float* z1 = zs + rr * H;
-  float* z2 = zs + (n + rr) * H;
-  float* z3 = zs + (2 * n + rr) * H;
-  __nv_bfloat16* h1 = hs + rr * H;
-  __nv_bfloat16* h2 = hs + (n + rr) * H;
-  __nv_bfloat16* h3 = hs + (2 * n + rr) * H;
+  // every thread's shared-memory writes and tensor-memory reads before the MMAs that thread 0 issues next
+  auto handover = [&]() {
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+  };
+  auto finished = [&]() {  // the MMAs committed last, or a wait that expired, for all threads alike
+    const bool w = mbar_wait(mb, parity);
+    parity ^= 1u;
+    ok = __syncthreads_and(w);
+    tc_fence_after();
+    return ok;
+  };
+  // one layer's activations: z (this thread's 32 columns) to h and, in place, g
+  auto activate = [&](float* z, float* h) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) gelu_both(z[i], h[i], z[i]);
+  };
+  auto store_tile = [&](__nv_bfloat16* tile, const float* v) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) store8(tile, r, c0 / 8 + q, v + q * 8);
+  };
+  // operand tile as MN-major: neighbouring 8-column groups 128 B apart, 8-row groups (K) 2048 B
+  auto mn = [&](const __nv_bfloat16* tile, int k) { return smem_desc(smem_u32(tile) + k * 4096, 2048, 128); };
+  auto kmaj = [&](const __nv_bfloat16* tile, int k) { return smem_desc(smem_u32(tile) + k * 256, 128, 2048); };
 
-  float x[IN];
-#pragma unroll
-  for (int j = 0; j < IN; ++j) x[j] = valid ? xn[row * IN + j] : 0.f;
   // ---- forward
-  for (int k8 = 0; k8 < H / 8; ++k8) {
-    float v[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int f = k8 * 8 + i;
-      float z = P.p[OFF_B1 + f];
-#pragma unroll
-      for (int j = 0; j < IN; ++j) z = fmaf(w1[f * IN + j], bf16r(x[j]), z);
-      if (valid) z1[f] = z;
-      v[i] = gelu(z);
-      if (valid) h1[f] = __float2bfloat16_rn(v[i]);
-    }
-    store8(ta, t, k8, v);
-  }
-  load_tile(tb, P.w2tc);
-  ok = tile_gemm(ta, tb, tmem, mb, parity);
-  if (ok) {
-    for (int c = 0; c < 4; ++c) {
-      float v[32];
-      tmem_ld32(lane_taddr(tmem) + c * 32, v);
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const int f = c * 32 + i;
-        const float z = v[i] + P.p[OFF_B2 + f];
-        if (valid) z2[f] = z;
-        v[i] = gelu(z);
-        if (valid) h2[f] = __float2bfloat16_rn(v[i]);
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) store8(ta, t, c * 4 + q, v + q * 8);
-    }
-    tc_fence_before();
-    __syncthreads();  // every warp has read the accumulator and the B tile is free
-    load_tile(tb, P.w3tc);
-    ok = tile_gemm(ta, tb, tmem, mb, parity);
-  }
-  float y[OUT];
-#pragma unroll
-  for (int j = 0; j < OUT; ++j) y[j] = b4[j];
-  if (ok) {
-    for (int c = 0; c < 4; ++c) {
-      float v[32];
-      tmem_ld32(lane_taddr(tmem) + c * 32, v);
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const int f = c * 32 + i;
-        const float z = v[i] + P.p[OFF_B3 + f];
-        if (valid) z3[f] = z;
-        const float hb = bf16r(gelu(z));
-        if (valid) h3[f] = __float2bfloat16_rn(hb);
-#pragma unroll
-        for (int j = 0; j < OUT; ++j) y[j] = fmaf(w4[j * H + f], hb, y[j]);
-      }
-    }
-  }
-  // ---- loss and output gradient
-  float lsum = 0.f;
-#pragma unroll
-  for (int j = 0; j < OUT; ++j) {
-    const float m = valid ? mask[row * OUT + j] : 0.f;
-    const float e = valid ? y[j] - yt[row * OUT + j] : 0.f;
-    lsum += m * e * e;
-    dys[t * OUT + j] = 2.f * m * e * inv_count;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-  if ((t & 31) == 0) red[t >> 5] = lsum;
-  tc_fence_before();
-  __syncthreads();
-  if (t == 0) atomicAdd(loss_sum, red[0] + red[1] + red[2] + red[3]);
-  // dW4, db4: thread t owns feature t
   {
-    float acc[OUT] = {0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int r = 0; r < TILE; ++r) {
-      const int64_t gr = (int64_t)blockIdx.x * TILE + r;
-      if (gr >= n) break;
-      const float h = __bfloat162float(hs[(2 * n + gr) * H + t]);
+    float z[32], h[32];
 #pragma unroll
-      for (int j = 0; j < OUT; ++j) acc[j] = fmaf(dys[r * OUT + j], h, acc[j]);
+    for (int i = 0; i < 32; ++i) {
+      const float4 w = *reinterpret_cast<const float4*>(w1 + (c0 + i) * IN);
+      z[i] = fmaf(w.w, x[3], fmaf(w.z, x[2], fmaf(w.y, x[1], fmaf(w.x, x[0], b123[c0 + i]))));
     }
+    activate(z, h);
+    tmem_st32(ta, z);
+    store_tile(h1, h);
+  }
+  handover();
+  if (t == 0) {
+    for (int k = 0; k < 8; ++k) mma_idesc(tm + 128, kmaj(h1, k), kmaj(w2, k), kIdesc, k > 0);
+    mma_commit(mb);
+  }
+  if (finished()) {
+    float z[32], h[32];
+    tmem_ld32(ta + 128, z);
 #pragma unroll
-    for (int j = 0; j < OUT; ++j) atomicAdd(grad + OFF_W4 + j * H + t, acc[j]);
-    if (t < OUT) {
-      float s = 0.f;
-      for (int r = 0; r < TILE; ++r) s += dys[r * OUT + t];
-      atomicAdd(grad + OFF_B4 + t, s);
+    for (int i = 0; i < 32; ++i) z[i] += b123[H + c0 + i];
+    activate(z, h);
+    tmem_st32(ta + 128, z);
+    store_tile(h2, h);
+    handover();
+    if (t == 0) {
+      for (int k = 0; k < 8; ++k) mma_idesc(tm + 256, kmaj(h2, k), kmaj(w3, k), kIdesc, k > 0);
+      mma_commit(mb);
     }
   }
-  // dz3 = (dy W4) * gelu'(z3): natural into ta, transposed into tt
-  for (int k8 = 0; k8 < H / 8; ++k8) {
-    float v[8];
+  // BF16 rows of h3, the 16-byte words of a row permuted by its low bits (no bank conflicts by row or by column)
+  auto h3_at = [&](int rr, int word) { return h3s + rr * 256 + ((word ^ (rr & 7)) << 4); };
+  if (ok && finished()) {
+    float z[32], h[32];
+    tmem_ld32(ta + 256, z);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int f = k8 * 8 + i;
-      float dh = 0.f;
+    for (int i = 0; i < 32; ++i) z[i] += b123[2 * H + c0 + i];
+    activate(z, h);
+    tmem_st32(ta + 256, z);
 #pragma unroll
-      for (int j = 0; j < OUT; ++j) dh = fmaf(dys[t * OUT + j], w4[j * H + f], dh);
-      const float dz = valid ? dh * gelu_grad(z3[f]) : 0.f;
-      v[i] = dz;
-      if (valid) atomicAdd(grad + OFF_B3 + f, dz);
-      tt[tc_offset(f, t)] = __float2bfloat16_rn(dz);
+    for (int q = 0; q < 4; ++q) {
+      __align__(16) __nv_bfloat162 b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) b[i] = __floats2bfloat162_rn(h[q * 8 + 2 * i], h[q * 8 + 2 * i + 1]);
+      *reinterpret_cast<int4*>(h3_at(r, c0 / 8 + q)) = *reinterpret_cast<int4*>(b);
     }
-    store8(ta, t, k8, v);
-  }
-  // h2 transposed into tb: dW3 = dz3^T h2 over the tile's rows
-  for (int f = 0; f < H; ++f) tb[tc_offset(f, t)] = valid ? h2[f] : __float2bfloat16_rn(0.f);
-  if (ok) ok = tile_gemm(tt, tb, tmem, mb, parity);
-  if (ok) {
-    for (int c = 0; c < 4; ++c) {
-      float v[32];
-      tmem_ld32(lane_taddr(tmem) + c * 32, v);
-#pragma unroll
-      for (int i = 0; i < 32; ++i) atomicAdd(grad + OFF_W3 + t * H + c * 32 + i, v[i]);
-    }
-    tc_fence_before();
     __syncthreads();
-    load_tile(tb, P.w3ttc);  // dh2 = dz3 W3
-    ok = tile_gemm(ta, tb, tmem, mb, parity);
-  }
-  if (ok) {
-    for (int c = 0; c < 4; ++c) {
-      float v[32];
-      tmem_ld32(lane_taddr(tmem) + c * 32, v);
+    // ---- output layer, loss and output gradient: one row per thread of the first four warps
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // count_kernel: mask sum, zeroed gradients
+    double cnt = 0.0;
+    for (int i = 0; i < kCountBlocks; ++i) cnt += part[i];
+    const float inv_count = cnt > 0.0 ? (float)(1.0 / cnt) : 0.f;
+    if (t < TILE) {
+      float y[OUT];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const int f = c * 32 + i;
-        const float dz = valid ? v[i] * gelu_grad(z2[f]) : 0.f;
-        v[i] = dz;
-        if (valid) atomicAdd(grad + OFF_B2 + f, dz);
-        tt[tc_offset(f, t)] = __float2bfloat16_rn(dz);
-      }
+      for (int j = 0; j < OUT; ++j) y[j] = P.p[OFF_B4 + j];
+      for (int q = 0; q < 16; ++q) {
+        const int4 b = *reinterpret_cast<const int4*>(h3_at(r, q));
+        const __nv_bfloat162* hb = reinterpret_cast<const __nv_bfloat162*>(&b);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) store8(ta, t, c * 4 + q, v + q * 8);
-    }
-    tc_fence_before();
-    __syncthreads();
-    for (int f = 0; f < H; ++f) tb[tc_offset(f, t)] = valid ? h1[f] : __float2bfloat16_rn(0.f);
-    ok = tile_gemm(tt, tb, tmem, mb, parity);  // dW2 = dz2^T h1
-  }
-  if (ok) {
-    for (int c = 0; c < 4; ++c) {
-      float v[32];
-      tmem_ld32(lane_taddr(tmem) + c * 32, v);
-#pragma unroll
-      for (int i = 0; i < 32; ++i) atomicAdd(grad + OFF_W2 + t * H + c * 32 + i, v[i]);
-    }
-    tc_fence_before();
-    __syncthreads();
-    load_tile(tb, P.w2ttc);  // dh1 = dz2 W2
-    ok = tile_gemm(ta, tb, tmem, mb, parity);
-  }
-  if (ok) {
-    for (int c = 0; c < 4; ++c) {
-      float v[32];
-      tmem_ld32(lane_taddr(tmem) + c * 32, v);
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const int f = c * 32 + i;
-        const float dz = valid ? v[i] * gelu_grad(z1[f]) : 0.f;
-        if (valid) {
-          atomicAdd(grad + OFF_B1 + f, dz);
-#pragma unroll
-          for (int j = 0; j < IN; ++j) atomicAdd(grad + OFF_W1 + f * IN + j, dz * bf16r(x[j]));
+        for (int i = 0; i < 8; ++i) {
+          const float hv = i & 1 ? __high2float(hb[i / 2]) : __low2float(hb[i / 2]);
+          const float4 w = *reinterpret_cast<const float4*>(w4 + (q * 8 + i) * 8);
+          y[0] = fmaf(w.x, hv, y[0]);
+          y[1] = fmaf(w.y, hv, y[1]);
+          y[2] = fmaf(w.z, hv, y[2]);
+          y[3] = fmaf(w.w, hv, y[3]);
+          y[4] = fmaf(w4[(q * 8 + i) * 8 + 4], hv, y[4]);
         }
       }
+      float lsum = 0.f;
+#pragma unroll
+      for (int j = 0; j < OUT; ++j) {
+        const float m = valid ? mask[row * OUT + j] : 0.f;
+        const float e = valid ? y[j] - yt[row * OUT + j] : 0.f;
+        lsum += m * e * e;
+        dys[r * 8 + j] = 2.f * m * e * inv_count;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+      if (lane == 0) atomicAdd(grad + N_PARAMS, lsum);
     }
+    __syncthreads();
+    // dW4, db4: feature f over a quarter of the rows
+    {
+      const int f = t & (H - 1), r0 = (t >> 7) * 32;
+      float acc[OUT] = {0.f, 0.f, 0.f, 0.f, 0.f}, s = 0.f;
+#pragma unroll 4
+      for (int rr = r0; rr < r0 + 32; ++rr) {
+        const float hv = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(h3_at(rr, f >> 3) + (f & 7) * 2));
+        const float4 d = *reinterpret_cast<const float4*>(dys + rr * 8);
+        const float d4 = dys[rr * 8 + 4];
+        acc[0] = fmaf(d.x, hv, acc[0]);
+        acc[1] = fmaf(d.y, hv, acc[1]);
+        acc[2] = fmaf(d.z, hv, acc[2]);
+        acc[3] = fmaf(d.w, hv, acc[3]);
+        acc[4] = fmaf(d4, hv, acc[4]);
+        if (f < OUT) s += dys[rr * 8 + f];
+      }
+#pragma unroll
+      for (int j = 0; j < OUT; ++j) atomicAdd(grad + OFF_W4 + j * H + f, acc[j]);
+      if (f < OUT) atomicAdd(grad + OFF_B4 + f, s);
+    }
+    // ---- backward: dz3 = (dy W4) * g3
+    {
+      float g[32];
+      tmem_ld32(ta + 256, g);
+      const float4 d = *reinterpret_cast<const float4*>(dys + r * 8);
+      const float d4 = dys[r * 8 + 4];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const float4 w = *reinterpret_cast<const float4*>(w4 + (c0 + i) * 8);
+        float dh = fmaf(d.x, w.x, 0.f);
+        dh = fmaf(d.y, w.y, dh);
+        dh = fmaf(d.z, w.z, dh);
+        dh = fmaf(d.w, w.w, dh);
+        dh = fmaf(d4, w4[(c0 + i) * 8 + 4], dh);
+        g[i] = valid ? dh * g[i] : 0.f;
+      }
+      store_tile(dz3, g);
+      atomicAdd(grad + OFF_B3 + c0 + lane, warp_column_sum(g));
+    }
+    handover();
+    if (t == 0) {  // dW3 = dz3^T h2 and dh2 = dz3 W3
+      for (int k = 0; k < 8; ++k) mma_idesc(tm + 256, kmaj(dz3, k), mn(w3, k), kIdescKMn, k > 0);
+      for (int k = 0; k < 8; ++k) mma_idesc(tm + 384, mn(dz3, k), mn(h2, k), kIdescMnMn, k > 0);
+      mma_commit(mb);
+    }
+  }
+  if (ok && finished()) {
+    {
+      float v[32], g[32];
+      tmem_ld32(ta + 256, v);
+      tmem_ld32(ta + 128, g);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = valid ? v[i] * g[i] : 0.f;
+      store_tile(dz2, v);
+      atomicAdd(grad + OFF_B2 + c0 + lane, warp_column_sum(v));
+      tmem_ld32(ta + 384, v);
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<float4*>(gw3 + r * kGradPitch + (c0 + 4 * q) * 4) =
+            make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    }
+    handover();
+    if (t == 0) {  // dh1 = dz2 W2 and dW2 = dz2^T h1
+      for (int k = 0; k < 8; ++k) mma_idesc(tm + 128, kmaj(dz2, k), mn(w2, k), kIdescKMn, k > 0);
+      for (int k = 0; k < 8; ++k) mma_idesc(tm + 384, mn(dz2, k), mn(h1, k), kIdescMnMn, k > 0);
+      mma_commit(mb);
+    }
+    if (t >= TRAIN_THREADS - TILE) {
+      const int o = t - (TRAIN_THREADS - TILE);
+      bulk_add_row(grad + OFF_W3 + o * H, gw3 + o * kGradPitch);
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // dz1 and dW2 are staged over it next
+    }
+    if (finished()) {
+      float v[32], g[32];
+      tmem_ld32(ta + 128, v);
+      tmem_ld32(ta, g);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {  // dz1 rows, their 16-byte words permuted like those of h3
+        float d[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[i] = valid ? v[4 * q + i] * g[4 * q + i] : 0.f;
+        *reinterpret_cast<float4*>(dz1s + r * 512 + (((c0 / 4 + q) ^ (r & 7)) << 4)) =
+            make_float4(d[0], d[1], d[2], d[3]);
+      }
+      tmem_ld32(ta + 384, v);
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<float4*>(gw2 + r * kGradPitch + (c0 + 4 * q) * 4) =
+            make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+      handover();
+      if (t >= TRAIN_THREADS - TILE) {
+        const int o = t - (TRAIN_THREADS - TILE);
+        bulk_add_row(grad + OFF_W2 + o * H, gw2 + o * kGradPitch);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      }
+      // dW1, db1: feature f over a quarter of the rows
+      const int f = t & (H - 1), r0 = (t >> 7) * 32;
+      float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f, s = 0.f;
+#pragma unroll 4
+      for (int rr = r0; rr < r0 + 32; ++rr) {
+        const float d = *reinterpret_cast<const float*>(dz1s + rr * 512 + (((f >> 2) ^ (rr & 7)) << 4) + (f & 3) * 4);
+        const float4 xr = *reinterpret_cast<const float4*>(xs + rr * IN);
+        a0 = fmaf(d, xr.x, a0);
+        a1 = fmaf(d, xr.y, a1);
+        a2 = fmaf(d, xr.z, a2);
+        a3 = fmaf(d, xr.w, a3);
+        s += d;
+      }
+      atomicAdd(grad + OFF_W1 + f * IN + 0, a0);
+      atomicAdd(grad + OFF_W1 + f * IN + 1, a1);
+      atomicAdd(grad + OFF_W1 + f * IN + 2, a2);
+      atomicAdd(grad + OFF_W1 + f * IN + 3, a3);
+      atomicAdd(grad + OFF_B1 + f, s);
+    }
+    if (t >= TRAIN_THREADS - TILE) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   if (!ok && t == 0) atomicExch(P.error, 1);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  tmem_free(tmem);
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tm));
 }
 
-// Adam on the FP32 master parameters (gradients zeroed afterwards).
-__global__ void adam_kernel(float* __restrict__ p, float* __restrict__ g, float* __restrict__ m,
-                            float* __restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N_PARAMS; i += gridDim.x * blockDim.x) {
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    p[i] -= lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-    g[i] = 0.f;
-  }
-}
+// The BF16 copies of the master parameters that the tensor cores read.
+struct Copies {
+  __nv_bfloat16 *w2tc, *w3tc, *w2h, *w3h, *w1tc, *w4tc, *b2t, *b3t;
+};
 
-// BF16 tensor-core copies and BF16-rounded narrow layers from the masters.
-__global__ void prepare_kernel(const float* __restrict__ p, float* __restrict__ w1r, float* __restrict__ w4r,
-                               __nv_bfloat16* __restrict__ w2tc, __nv_bfloat16* __restrict__ w3tc,
-                               __nv_bfloat16* __restrict__ w2ttc, __nv_bfloat16* __restrict__ w3ttc,
-                               __nv_bfloat16* __restrict__ w1tc, __nv_bfloat16* __restrict__ w4tc,
-                               __nv_bfloat16* __restrict__ b2t, __nv_bfloat16* __restrict__ b3t,
-                               __nv_bfloat16* __restrict__ w2h, __nv_bfloat16* __restrict__ w3h) {
-  // a bias as two BF16 columns, hi + lo = b to about 2^-16 relative
-  auto split = [](float b, int part) {
-    const __nv_bfloat16 hi = __float2bfloat16_rn(b);
-    return part == 0 ? hi : __float2bfloat16_rn(b - __bfloat162float(hi));
+// Writes the copies of parameter i, of value v (the tiles' padding is zeroed
+// once, at creation).
+__device__ __forceinline__ void write_copies(const Copies& C, int i, float v) {
+  auto split = [&](__nv_bfloat16* tile, int o, int k) {  // a bias as two BF16 columns, hi + lo = b to about 2^-16 relative
+    const __nv_bfloat16 hi = __float2bfloat16_rn(v);
+    tile[tc16_offset(o, k)] = hi;
+    tile[tc16_offset(o, k + 1)] = __float2bfloat16_rn(v - __bfloat162float(hi));
   };
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < H * 16; i += gridDim.x * blockDim.x) {
-    const int o = i / 16, k = i % 16;  // layer 1: rows = out (128), K = in (4 of 16), then b1 hi, lo
-    w1tc[tc16_offset(o, k)] = k < IN ? __float2bfloat16_rn(p[OFF_W1 + o * IN + k])
-                              : k < IN + 2 ? split(p[OFF_B1 + o], k - IN) : __float2bfloat16_rn(0.f);
-    b2t[tc16_offset(o, k)] = k < 2 ? split(p[OFF_B2 + o], k) : __float2bfloat16_rn(0.f);
-    b3t[tc16_offset(o, k)] = k < 2 ? split(p[OFF_B3 + o], k) : __float2bfloat16_rn(0.f);
-    const int r = i / H, kk = i % H;   // layer 4: rows = out (5 of 16), K = in (128); takes 2 GELU
-    w4tc[tc_offset(r, kk)] = __float2bfloat16_rn(r < OUT ? 0.5f * p[OFF_W4 + r * H + kk] : 0.f);
+  if (i < OFF_B1) {
+    C.w1tc[tc16_offset(i / IN, i % IN)] = __float2bfloat16_rn(v);
+  } else if (i < OFF_W2) {
+    split(C.w1tc, i - OFF_B1, IN);
+  } else if (i < OFF_B2) {
+    const int at = tc_offset((i - OFF_W2) / H, (i - OFF_W2) % H);
+    C.w2tc[at] = __float2bfloat16_rn(v);
+    C.w2h[at] = __float2bfloat16_rn(0.5f * v);
+  } else if (i < OFF_W3) {
+    split(C.b2t, i - OFF_B2, 0);
+  } else if (i < OFF_B3) {
+    const int at = tc_offset((i - OFF_W3) / H, (i - OFF_W3) % H);
+    C.w3tc[at] = __float2bfloat16_rn(v);
+    C.w3h[at] = __float2bfloat16_rn(0.5f * v);
+  } else if (i < OFF_W4) {
+    split(C.b3t, i - OFF_B3, 0);
+  } else if (i < OFF_B4) {
+    C.w4tc[tc_offset((i - OFF_W4) / H, (i - OFF_W4) % H)] = __float2bfloat16_rn(0.5f * v);
   }
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < H * H; i += gridDim.x * blockDim.x) {
-    const int o = i / H, k = i % H;
-    w2tc[tc_offset(o, k)] = __float2bfloat16_rn(p[OFF_W2 + i]);   // B of h W2^T: rows = out, K = in
-    w3tc[tc_offset(o, k)] = __float2bfloat16_rn(p[OFF_W3 + i]);
-    w2ttc[tc_offset(k, o)] = __float2bfloat16_rn(p[OFF_W2 + i]);  // B of dz W2: rows = in, K = out
-    w3ttc[tc_offset(k, o)] = __float2bfloat16_rn(p[OFF_W3 + i]);
-    w2h[tc_offset(o, k)] = __float2bfloat16_rn(0.5f * p[OFF_W2 + i]);
-    w3h[tc_offset(o, k)] = __float2bfloat16_rn(0.5f * p[OFF_W3 + i]);
-    if (i < H * IN) w1r[i] = bf16r(p[OFF_W1 + i]);
-    if (i < OUT * H) w4r[i] = bf16r(p[OFF_W4 + i]);
-  }
+}
+
+// Adam on the FP32 master parameters, and their BF16 copies.
+__global__ void __launch_bounds__(256) adam_kernel(float* __restrict__ p, const float* __restrict__ g,
+                                                   float* __restrict__ m, float* __restrict__ v, const Copies C,
+                                                   float lr, float b1, float b2, float eps, float c1, float c2) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N_PARAMS) return;
+  const float gi = g[i];
+  const float mi = b1 * m[i] + (1.f - b1) * gi;
+  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+  m[i] = mi;
+  v[i] = vi;
+  const float w = p[i] - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+  p[i] = w;
+  write_copies(C, i, w);
+}
+
+__global__ void __launch_bounds__(256) prepare_kernel(const float* __restrict__ p, const Copies C) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < N_PARAMS) write_copies(C, i, p[i]);
 }
 
 // One 128 x 128 x 128 GEMM through the tensor-core path (descriptor self-test):
@@ -884,7 +1042,7 @@ __global__ void gamma_fit_kernel(const double* __restrict__ hist, int64_t n, int
 }
 
 constexpr size_t kInferSmem = (2 + kGroups) * TILE_BYTES + 5 * H * 16 * 2 + (8 + 24) * 4 + 8 * kGroups + 16;
-constexpr size_t kTrainSmem = 3 * TILE_BYTES + (H * IN + OUT * H + 8 + TILE * OUT + 8) * 4 + 16 + 16;
+constexpr size_t kTrainSmem = 6 * TILE_BYTES + (H * IN + H * 8 + TILE * 8 + TILE * IN + 3 * H) * 4 + 16;
 constexpr size_t kTestSmem = 2 * TILE_BYTES + 32;
 
 }  // namespace mlp
@@ -896,18 +1054,11 @@ struct pp_mlp {
   int sm_count = 0;
   std::mutex mu;
   float* d_params = nullptr;  // N_PARAMS
-  float* d_grad = nullptr;
+  float* d_grad = nullptr;  // kBack words: gradients, loss sum, error flag, mask sums
   float* d_m = nullptr;
   float* d_v = nullptr;
-  float* d_w1r = nullptr;
-  float* d_w4r = nullptr;
-  __nv_bfloat16* d_tc = nullptr;  // 6 tiles of 128 x 128, then 4 of 128 x 16
+  __nv_bfloat16* d_tc = nullptr;  // 4 tiles of 128 x 128, then 4 of 128 x 16
   float* d_norm = nullptr;        // 18 (+ pad)
-  int* d_error = nullptr;
-  float* d_loss = nullptr;
-  float* d_zs = nullptr;
-  __nv_bfloat16* d_hs = nullptr;
-  int64_t scratch_rows = 0;
   int64_t step = 0;
   std::string err;
 };
@@ -927,26 +1078,26 @@ struct Guard {
 mlp::DevParams dev_params(pp_mlp* m) {
   mlp::DevParams P;
   P.p = m->d_params;
-  P.w1r = m->d_w1r;
-  P.w4r = m->d_w4r;
   P.w2tc = m->d_tc;
   P.w3tc = m->d_tc + mlp::TILE * mlp::H;
-  P.w2ttc = m->d_tc + 2 * mlp::TILE * mlp::H;
-  P.w2h = m->d_tc + 4 * mlp::TILE * mlp::H;
-  P.w3h = m->d_tc + 5 * mlp::TILE * mlp::H;
-  P.w1tc = m->d_tc + 6 * mlp::TILE * mlp::H;
+  P.w2h = m->d_tc + 2 * mlp::TILE * mlp::H;
+  P.w3h = m->d_tc + 3 * mlp::TILE * mlp::H;
+  P.w1tc = m->d_tc + 4 * mlp::TILE * mlp::H;
   P.w4tc = P.w1tc + mlp::H * 16;
-  P.w3ttc = m->d_tc + 3 * mlp::TILE * mlp::H;
   P.norm = m->d_norm;
-  P.error = m->d_error;
+  P.error = reinterpret_cast<int*>(m->d_grad + mlp::N_PARAMS + 1);
   return P;
 }
 
-cudaError_t prepare(pp_mlp* m, cudaStream_t s) {
+mlp::Copies copies(pp_mlp* m) {
   __nv_bfloat16* t = m->d_tc;
   constexpr int T = mlp::TILE * mlp::H, S = mlp::H * 16;
-  mlp::prepare_kernel<<<64, 256, 0, s>>>(m->d_params, m->d_w1r, m->d_w4r, t, t + T, t + 2 * T, t + 3 * T, t + 6 * T,
-                                         t + 6 * T + S, t + 6 * T + 2 * S, t + 6 * T + 3 * S, t + 4 * T, t + 5 * T);
+  return mlp::Copies{t, t + T, t + 2 * T, t + 3 * T, t + 4 * T, t + 4 * T + S, t + 4 * T + 2 * S, t + 4 * T + 3 * S};
+}
+constexpr int kParamBlocks = (mlp::N_PARAMS + 255) / 256;
+
+cudaError_t prepare(pp_mlp* m, cudaStream_t s) {
+  mlp::prepare_kernel<<<kParamBlocks, 256, 0, s>>>(m->d_params, copies(m));
   pp::count_launches(1);
   return cudaGetLastError();
 }
@@ -974,14 +1125,13 @@ pp_status pp_mlp_create(int device, uint64_t seed, pp_mlp** out) {
   cudaGetDeviceProperties(&prop, device);
   m->sm_count = prop.multiProcessorCount;
   cudaError_t e;
-  if ((e = cudaMalloc(&m->d_params, mlp::N_PARAMS * 4)) || (e = cudaMalloc(&m->d_grad, mlp::N_PARAMS * 4)) ||
+  constexpr size_t kTcBytes = 4 * mlp::TILE_BYTES + 4 * mlp::H * 16 * 2;
+  if ((e = cudaMalloc(&m->d_params, mlp::N_PARAMS * 4)) || (e = cudaMalloc(&m->d_grad, mlp::kBack * 4)) ||
       (e = cudaMalloc(&m->d_m, mlp::N_PARAMS * 4)) || (e = cudaMalloc(&m->d_v, mlp::N_PARAMS * 4)) ||
-      (e = cudaMalloc(&m->d_w1r, mlp::H * mlp::IN * 4)) || (e = cudaMalloc(&m->d_w4r, mlp::OUT * mlp::H * 4)) ||
-      (e = cudaMalloc(&m->d_tc, 6 * mlp::TILE_BYTES + 4 * mlp::H * 16 * 2)) || (e = cudaMalloc(&m->d_norm, 32 * 4)) ||
-      (e = cudaMalloc(&m->d_error, 16)) || (e = cudaMalloc(&m->d_loss, 16))) {
+      (e = cudaMalloc(&m->d_tc, kTcBytes)) || (e = cudaMalloc(&m->d_norm, 32 * 4))) {
     cudaGetLastError();
-    for (void* b : {(void*)m->d_params, (void*)m->d_grad, (void*)m->d_m, (void*)m->d_v, (void*)m->d_w1r,
-                    (void*)m->d_w4r, (void*)m->d_tc, (void*)m->d_norm, (void*)m->d_error, (void*)m->d_loss})
+    for (void* b : {(void*)m->d_params, (void*)m->d_grad, (void*)m->d_m, (void*)m->d_v, (void*)m->d_tc,
+                    (void*)m->d_norm})
       if (b) cudaFree(b);
     delete m;
     return e == cudaErrorMemoryAllocation ? PP_ERR_OOM : PP_ERR_CUDA;
@@ -1008,9 +1158,9 @@ pp_status pp_mlp_create(int device, uint64_t seed, pp_mlp** out) {
   for (int j = 0; j < 4; ++j) norm[4 + j] = 1.f;
   for (int j = 0; j < 5; ++j) norm[13 + j] = 1.f;
   if ((e = cudaMemcpy(m->d_params, p.data(), mlp::N_PARAMS * 4, cudaMemcpyHostToDevice)) ||
-      (e = cudaMemset(m->d_grad, 0, mlp::N_PARAMS * 4)) || (e = cudaMemset(m->d_m, 0, mlp::N_PARAMS * 4)) ||
+      (e = cudaMemset(m->d_grad, 0, mlp::kBack * 4)) || (e = cudaMemset(m->d_m, 0, mlp::N_PARAMS * 4)) ||
       (e = cudaMemset(m->d_v, 0, mlp::N_PARAMS * 4)) || (e = cudaMemcpy(m->d_norm, norm, 128, cudaMemcpyHostToDevice)) ||
-      (e = cudaMemset(m->d_error, 0, 16)) || (e = prepare(m, nullptr)) || (e = cudaDeviceSynchronize())) {
+      (e = cudaMemset(m->d_tc, 0, kTcBytes)) || (e = prepare(m, nullptr)) || (e = cudaDeviceSynchronize())) {
     cudaGetLastError();
     pp_mlp_destroy(m);
     return PP_ERR_CUDA;
@@ -1026,9 +1176,8 @@ void pp_mlp_destroy(pp_mlp* m) {
   if (!m) return;
   Guard g(m->device);
   cudaDeviceSynchronize();
-  for (void* p : {(void*)m->d_params, (void*)m->d_grad, (void*)m->d_m, (void*)m->d_v, (void*)m->d_w1r,
-                  (void*)m->d_w4r, (void*)m->d_tc, (void*)m->d_norm, (void*)m->d_error, (void*)m->d_loss,
-                  (void*)m->d_zs, (void*)m->d_hs})
+  for (void* p : {(void*)m->d_params, (void*)m->d_grad, (void*)m->d_m, (void*)m->d_v, (void*)m->d_tc,
+                  (void*)m->d_norm})
     if (p) cudaFree(p);
   delete m;
 }
@@ -1101,51 +1250,36 @@ pp_status pp_mlp_train_step(pp_mlp* m, const float* d_xn, const float* d_yt, con
   std::lock_guard<std::mutex> lk(m->mu);
   Guard g(m->device);
   cudaError_t e;
-  if (n > m->scratch_rows) {
-    if (m->d_zs) cudaFree(m->d_zs);
-    if (m->d_hs) cudaFree(m->d_hs);
-    m->d_zs = nullptr;
-    m->d_hs = nullptr;
-    m->scratch_rows = 0;
-    if ((e = cudaMalloc(&m->d_zs, (size_t)3 * n * mlp::H * 4)) ||
-        (e = cudaMalloc(&m->d_hs, (size_t)3 * n * mlp::H * 2))) {
-      cudaGetLastError();
-      return fail(m, PP_ERR_OOM, "pp_mlp_train_step: scratch");
-    }
-    m->scratch_rows = n;
-  }
-  // mask count for the mean
-  std::vector<float> hmask((size_t)n * mlp::OUT);
-  if ((e = cudaMemcpy(hmask.data(), d_mask, hmask.size() * 4, cudaMemcpyDeviceToHost)))
-    return fail(m, PP_ERR_CUDA, "pp_mlp_train_step: mask");
-  double cnt = 0;
-  for (float v : hmask) cnt += v;
-  const float inv = cnt > 0 ? (float)(1.0 / cnt) : 0.f;
-  if ((e = cudaMemset(m->d_loss, 0, 4)) || (e = cudaMemset(m->d_grad, 0, mlp::N_PARAMS * 4)))
-    return fail(m, PP_ERR_CUDA, "pp_mlp_train_step: memset");
-  const int grid = (int)((n + mlp::TILE - 1) / mlp::TILE);
-  mlp::train_kernel<<<grid, mlp::THREADS, mlp::kTrainSmem>>>(dev_params(m), d_xn, d_yt, d_mask, n, inv, m->d_grad,
-                                                              m->d_loss, m->d_zs, m->d_hs);
+  const int64_t tiles = (n + mlp::TILE - 1) / mlp::TILE;
+  if (tiles > INT32_MAX) return fail(m, PP_ERR_ARG, "pp_mlp_train_step: too many rows");
+  double* part = reinterpret_cast<double*>(m->d_grad + mlp::kPartAt);
+  mlp::count_kernel<<<mlp::kCountBlocks, 256>>>(d_mask, n * mlp::OUT, m->d_grad, part);
   pp::count_launches(1);
-  if ((e = cudaGetLastError())) return fail(m, PP_ERR_CUDA, std::string("train: ") + cudaGetErrorString(e));
-  if (grad_out && (e = cudaMemcpy(grad_out, m->d_grad, mlp::N_PARAMS * 4, cudaMemcpyDeviceToHost)))
-    return fail(m, PP_ERR_CUDA, "pp_mlp_train_step: grads");
+  if ((e = cudaGetLastError()) ||
+      (e = pp::launch_dependent(mlp::train_kernel, (int)tiles, mlp::TRAIN_THREADS, mlp::kTrainSmem, nullptr,
+                                dev_params(m), d_xn, d_yt, d_mask, n, part, m->d_grad)))
+    return fail(m, PP_ERR_CUDA, std::string("train: ") + cudaGetErrorString(e));
   if (lr > 0.f) {
     m->step += 1;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = (float)(1.0 / (1.0 - std::pow((double)b1, (double)m->step)));
     const float c2 = (float)(1.0 / (1.0 - std::pow((double)b2, (double)m->step)));
-    mlp::adam_kernel<<<64, 256>>>(m->d_params, m->d_grad, m->d_m, m->d_v, lr, b1, b2, 1e-8f, c1, c2);
-    pp::count_launches(1);
-    if ((e = prepare(m, nullptr))) return fail(m, PP_ERR_CUDA, "prepare");
+    if ((e = pp::launch_dependent(mlp::adam_kernel, kParamBlocks, 256, 0, nullptr, m->d_params, m->d_grad, m->d_m,
+                                  m->d_v, copies(m), lr, b1, b2, 1e-8f, c1, c2)))
+      return fail(m, PP_ERR_CUDA, std::string("adam: ") + cudaGetErrorString(e));
   }
-  float loss = 0.f;
-  int errflag = 0;
-  if ((e = cudaMemcpy(&loss, m->d_loss, 4, cudaMemcpyDeviceToHost)) ||
-      (e = cudaMemcpy(&errflag, m->d_error, 4, cudaMemcpyDeviceToHost)))
+  float back[mlp::kBack - mlp::N_PARAMS];  // loss sum, error flag, mask sums
+  if ((grad_out && (e = cudaMemcpyAsync(grad_out, m->d_grad, mlp::N_PARAMS * 4, cudaMemcpyDeviceToHost, nullptr))) ||
+      (e = cudaMemcpyAsync(back, m->d_grad + mlp::N_PARAMS, sizeof back, cudaMemcpyDeviceToHost, nullptr)) ||
+      (e = cudaStreamSynchronize(nullptr)))
     return fail(m, PP_ERR_CUDA, std::string("train: ") + cudaGetErrorString(e));
+  int errflag;
+  std::memcpy(&errflag, back + 1, 4);
   if (errflag) return fail(m, PP_ERR_TIMEOUT, "tensor-core wait expired");
-  if (loss_out) *loss_out = (float)(loss * inv);
+  double sums[mlp::kCountBlocks], cnt = 0.0;
+  std::memcpy(sums, back + (mlp::kPartAt - mlp::N_PARAMS), sizeof sums);
+  for (double v : sums) cnt += v;
+  if (loss_out) *loss_out = (float)(back[0] * (cnt > 0.0 ? (float)(1.0 / cnt) : 0.f));
   return PP_OK;
 }
 
