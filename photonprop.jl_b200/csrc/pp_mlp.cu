@@ -938,23 +938,26 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_test_kernel(const __nv_bfloat
 // Two-component Gamma mixture w G(a1, theta) + (1 - w) G(a2, theta) fitted by
 // weighted EM to each pair's arrival-time histogram, as a function of the
 // time residual t - t_shift (bins with a positive residual only; the reference
-// fits a single Gamma to the time residual, src/modelling.jl:52-79).  One warp
-// per pair.  M step: theta = sum_k S1_k / sum_k a_k S0_k, then psi(a_k) =
-// SL_k / S0_k - ln theta solved by Newton (psi and psi' from their asymptotic
-// series after upward recurrence).  Output per pair: w, a1 <= a2, theta,
-// mean log-likelihood per weight; NaNs when the histogram is empty.
-using ppsf::digamma_d;
-using ppsf::trigamma_d;
-
-// a with psi(a) = y (Minka's initialisation, Newton steps).
-__device__ double inv_digamma(double y) {
-  double a = y >= -2.22 ? exp(y) + 0.5 : -1.0 / (y + 0.5772156649015329);
-  for (int i = 0; i < 8; ++i) {
-    a -= (digamma_d(a) - y) / trigamma_d(a);
-    if (a < 1e-3) a = 1e-3;
-  }
-  return a;
-}
+// fits a single Gamma to the time residual, src/modelling.jl:52-79).
+// M step: theta = sum_k S1_k / sum_k a_k S0_k, then psi(a_k) =
+// SL_k / S0_k - ln theta solved by Newton, three times.  Output per pair: w,
+// a1 <= a2, theta, mean log-likelihood per weight; NaNs when the histogram is
+// empty.
+//
+// A warp fits up to 16 pairs together.  Their filled bins (weight, time, log
+// time) are gathered once into the warp's part of shared memory.  E step: the
+// warp walks one pair's bins after the other; the two densities share
+// t / theta, so their ratio takes one exponential, and the log-likelihood
+// one logarithm more, in the last iteration only.  M step: one lane per
+// (pair, component).  Bins that do not fit (a first pair of more than
+// kMixEntries filled bins) are read from the histogram again each time.
+//
+// Bound by FP64 issue.  With one pair per warp, every lane did the same 48
+// digamma and trigamma evaluations per iteration: 20,000 pairs of 1000 bins
+// (60 iterations) took 36.1 ms, now 3.8 ms (issue 50 % of active cycles, FP64
+// pipe 35 %, 16 warps per SM).
+constexpr int kMixWarps = 16, kMixEntries = 768, kMixPairs = 16;
+constexpr size_t kMixSmem = (size_t)kMixWarps * kMixEntries * (2 * sizeof(double) + sizeof(uint16_t));
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -962,82 +965,209 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-__global__ void gamma_fit_kernel(const double* __restrict__ hist, int64_t n, int bins, float t0, float bw,
-                                 const float* __restrict__ tshift, float* __restrict__ out, int iters) {
-  const int64_t pair = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (pair >= n) return;  // whole warps exit together
-  const double* h = hist + pair * bins;
-  const double ts = tshift[pair];
-  // moments for the initial guess
-  double s0 = 0, s1 = 0, s2 = 0;
-  for (int b = lane; b < bins; b += 32) {
-    const double t = t0 + (b + 0.5) * bw - ts;
-    if (t > 0 && h[b] > 0) {
-      s0 += h[b];
-      s1 += h[b] * t;
-      s2 += h[b] * t * t;
+// a >= 1e-3 with psi(a) = y: Newton from the last solution, or, where that is
+// far off, from Minka's initial value.  psi is concave, so from the second
+// step on the iterates rise to the root; their error is squared by each step,
+// so a step of 1e-8 leaves none that FP64 holds.  All lanes of the warp call.
+__device__ double inv_digamma(double y, double a, bool active) {
+  for (int i = 0; i < 24; ++i) {
+    double f, f1;
+    ppsf::psi_both(a, f, f1);
+    double n = a - (f - y) / f1;
+    if (i == 0 && !(n > 0.5 * a && n < 2.0 * a)) n = y >= -2.22 ? exp(y) + 0.5 : -1.0 / (y + 0.5772156649015329);
+    n = n < 1e-3 ? 1e-3 : n;
+    const bool moving = active && fabs(n - a) > 1e-8 * a;
+    a = n;
+    if (!__any_sync(0xffffffffu, moving)) break;
+  }
+  return a;
+}
+
+__global__ void __launch_bounds__(kMixWarps * 32, 1) gamma_fit_kernel(const double* __restrict__ hist, int64_t n, int bins,
+                                                                     float t0, float bw,
+                                                                     const float* __restrict__ tshift,
+                                                                     float* __restrict__ out, int iters) {
+  extern __shared__ double mix_smem[];
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // the filled bins: weight, log time, bin (a pair's bins from 65536 on are not gathered)
+  double* const eh = mix_smem + (size_t)warp * kMixEntries * 2;
+  double* const el = eh + kMixEntries;
+  uint16_t* const eb = reinterpret_cast<uint16_t*>(mix_smem + (size_t)kMixWarps * kMixEntries * 2) + warp * kMixEntries;
+  // the block's pairs are blockIdx.x + i gridDim.x; its warps take them from a
+  // counter, at most a warp's share of what is left at a time
+  __shared__ unsigned taken;
+  if (threadIdx.x == 0) taken = 0;
+  __syncthreads();
+  const int64_t mine = (n - blockIdx.x + gridDim.x - 1) / gridDim.x;
+  auto take = [&]() {
+    unsigned i = 0;
+    if (lane == 0) i = atomicAdd(&taken, 1u);
+    return (int64_t)__shfl_sync(kAll, i, 0);
+  };
+  int64_t next = take();
+  while (next < mine) {
+    const int share = (int)min((int64_t)kMixPairs, (mine - next + kMixWarps - 1) / kMixWarps);
+    // this lane's pair (lane / 2) and component (lane % 2; 0 is the one with the smaller start value)
+    int64_t pair = -1;
+    int first = 0, count = 0, rest = bins;  // entries in shared memory; bins from `rest` on are read again
+    double s0 = 0, a = 1, w = 0.5, th = 1;
+    int used = 0, m = 0;
+    for (; m < share && next < mine; ++m, next = take()) {
+      const int64_t row = blockIdx.x + next * gridDim.x;
+      const double* h = hist + row * bins;
+      const double ts = tshift[row];
+      double p0 = 0, p1 = 0, p2 = 0;
+      int k = 0, b0 = 0, stop = bins;
+      for (; b0 < bins; b0 += 32) {
+        const int b = b0 + lane;
+        const double hb = b < bins ? h[b] : 0.0, t = t0 + (b + 0.5) * bw - ts;
+        const bool in = t > 0 && hb > 0;
+        const unsigned ball = __ballot_sync(kAll, in);
+        if (!ball) continue;
+        if (in) {
+          p0 += hb;
+          p1 += hb * t;
+          p2 += hb * t * t;
+        }
+        if (stop < bins || used + k + __popc(ball) > kMixEntries || b0 > 65535 - 32) {
+          stop = min(stop, b0);
+          if (m > 0) break;  // the pair opens the next round
+          continue;
+        }
+        if (in) {
+          const int at = used + k + __popc(ball & ((1u << lane) - 1u));
+          eh[at] = hb;
+          el[at] = log(t);
+          eb[at] = (uint16_t)b;
+        }
+        k += __popc(ball);
+      }
+      if (m > 0 && stop < bins) break;
+      p0 = warp_sum(p0);
+      p1 = warp_sum(p1);
+      p2 = warp_sum(p2);
+      if ((lane >> 1) == m) {
+        pair = row;
+        first = used;
+        count = k;
+        rest = stop;
+        s0 = p0;
+        const double mean = p1 / p0, v = fmax(p2 / p0 - mean * mean, 1e-6 * mean * mean + 1e-12);
+        const double a0 = fmax(mean * mean / v, 0.05);
+        a = (lane & 1) ? 2.0 * a0 : fmax(0.5 * a0, 0.02);
+        th = v / mean;
+      }
+      used += k;
     }
-  }
-  s0 = warp_sum(s0);
-  s1 = warp_sum(s1);
-  s2 = warp_sum(s2);
-  float* o = out + pair * 5;
-  if (!(s0 > 0)) {
-    if (lane < 5) o[lane] = __int_as_float(0x7fc00000);
-    return;
-  }
-  const double m = s1 / s0, v = fmax(s2 / s0 - m * m, 1e-6 * m * m + 1e-12);
-  const double a0 = fmax(m * m / v, 0.05);
-  double w = 0.5, a1 = fmax(0.5 * a0, 0.02), a2 = 2.0 * a0, th = v / m;
-  double ll = 0;
-  for (int it = 0; it < iters; ++it) {
-    const double lw1 = log(w), lw2 = log1p(-w), lth = log(th);
-    const double c1 = lw1 - a1 * lth - lgamma(a1), c2 = lw2 - a2 * lth - lgamma(a2);
-    double S0a = 0, S1a = 0, SLa = 0, S0b = 0, S1b = 0, SLb = 0, L = 0;
-    for (int b = lane; b < bins; b += 32) {
-      const double t = t0 + (b + 0.5) * bw - ts;
-      const double hb = h[b];
-      if (!(t > 0) || !(hb > 0)) continue;
-      const double lt = log(t);
-      const double p1 = c1 + (a1 - 1) * lt - t / th, p2 = c2 + (a2 - 1) * lt - t / th;
-      const double mx = fmax(p1, p2);
-      const double e1 = exp(p1 - mx), e2 = exp(p2 - mx);
-      const double r1 = e1 / (e1 + e2);
-      L += hb * (mx + log(e1 + e2));
-      S0a += hb * r1;
-      S1a += hb * r1 * t;
-      SLa += hb * r1 * lt;
-      S0b += hb * (1 - r1);
-      S1b += hb * (1 - r1) * t;
-      SLb += hb * (1 - r1) * lt;
+    __syncwarp();
+    const bool live = pair >= 0 && s0 > 0;
+    if (!live) a = th = 1.0;  // harmless values for the lanes without a fit
+    double ll = 0;
+#pragma unroll 1
+    for (int it = 0; it < iters; ++it) {
+      const double lth = log(th), lw = (lane & 1) ? log1p(-w) : log(w);
+      const double c = lw - a * lth - lgamma(a);
+      const double cd = c - __shfl_xor_sync(kAll, c, 1), ad = a - __shfl_xor_sync(kAll, a, 1);
+      double S0 = 0, S1 = 0, SL = 0;  // this lane's component
+#pragma unroll 1
+      for (int p = 0; p < m; ++p) {
+        // log ratio of component 1's density to component 2's: da lt + dc (even lanes hold component 1)
+        const double dc = __shfl_sync(kAll, cd, 2 * p), da = __shfl_sync(kAll, ad, 2 * p);
+        const int f0 = __shfl_sync(kAll, first, 2 * p), k = __shfl_sync(kAll, count, 2 * p);
+        const int stop = __shfl_sync(kAll, rest, 2 * p);
+        const int64_t row = __shfl_sync(kAll, pair, 2 * p);
+        const double ts = tshift[row];
+        double q0 = 0, q1 = 0, q2 = 0, r0 = 0, r1 = 0, r2 = 0;
+        auto add = [&](double hb, double t, double lt) {
+          const double d = fma(da, lt, dc);
+          const double e = exp(-fabs(d)), v = 1.0 / (1.0 + e);
+          const double f = d > 0 ? v : e * v;  // component 1's share
+          // 1 - f, which is 0 once component 2 falls below the rounding of 1:
+          // its parameters then stay as they are
+          const double x = hb * f, y = hb * (1.0 - f);
+          q0 += x;
+          q1 = fma(x, t, q1);
+          q2 = fma(x, lt, q2);
+          r0 += y;
+          r1 = fma(y, t, r1);
+          r2 = fma(y, lt, r2);
+        };
+#pragma unroll 2
+        for (int i = f0 + lane; i < f0 + k; i += 32) add(eh[i], t0 + (eb[i] + 0.5) * bw - ts, el[i]);
+        if (stop < bins) {  // what did not fit
+          const double* h = hist + row * bins;
+#pragma unroll 1
+          for (int b = stop + lane; b < bins; b += 32) {
+            const double hb = h[b], t = t0 + (b + 0.5) * bw - ts;
+            if (t > 0 && hb > 0) add(hb, t, log(t));
+          }
+        }
+        // even lanes sum component 1, odd lanes component 2
+        const bool odd = lane & 1;
+        double u0 = odd ? r0 : q0, u1 = odd ? r1 : q1, u2 = odd ? r2 : q2;
+        u0 += __shfl_xor_sync(kAll, odd ? q0 : r0, 1);
+        u1 += __shfl_xor_sync(kAll, odd ? q1 : r1, 1);
+        u2 += __shfl_xor_sync(kAll, odd ? q2 : r2, 1);
+#pragma unroll
+        for (int o = 2; o < 32; o <<= 1) {
+          u0 += __shfl_xor_sync(kAll, u0, o);
+          u1 += __shfl_xor_sync(kAll, u1, o);
+          u2 += __shfl_xor_sync(kAll, u2, o);
+        }
+        if ((lane >> 1) == p) {
+          S0 = u0;
+          S1 = u1;
+          SL = u2;
+        }
+      }
+      if (it == iters - 1) {  // the log-likelihood, of the parameters that this iteration began with
+#pragma unroll 1
+        for (int p = 0; p < m; ++p) {
+          const double dc = __shfl_sync(kAll, cd, 2 * p), da = __shfl_sync(kAll, ad, 2 * p);
+          const double c2 = __shfl_sync(kAll, c, 2 * p + 1), a2 = __shfl_sync(kAll, a, 2 * p + 1);
+          const double rth = 1.0 / __shfl_sync(kAll, th, 2 * p);
+          const int64_t row = __shfl_sync(kAll, pair, 2 * p);
+          const double* h = hist + row * bins;
+          const double ts = tshift[row];
+          double L = 0;
+#pragma unroll 1
+          for (int b = lane; b < bins; b += 32) {
+            const double hb = h[b], t = t0 + (b + 0.5) * bw - ts;
+            if (!(t > 0) || !(hb > 0)) continue;
+            const double lt = log(t), d = fma(da, lt, dc);
+            L += hb * (fma(a2 - 1.0, lt, c2) - t * rth + fmax(d, 0.0) + log1p(exp(-fabs(d))));
+          }
+          L = warp_sum(L);
+          if ((lane >> 1) == p) ll = L / s0;
+        }
+      }
+      const double o0 = __shfl_xor_sync(kAll, S0, 1);
+      const double S1t = S1 + __shfl_xor_sync(kAll, S1, 1);
+      const double wa = (lane & 1) ? o0 : S0, wb = (lane & 1) ? S0 : o0;
+      if (live) w = fmin(fmax(wa / (wa + wb), 1e-4), 1 - 1e-4);
+      const bool solve = live && S0 > 0;
+#pragma unroll 1
+      for (int j = 0; j < 3; ++j) {
+        const double v = a * S0, vt = v + __shfl_xor_sync(kAll, v, 1);
+        if (live) th = S1t / vt;
+        const double y = solve ? SL / S0 - log(th) : 0.0;
+        const double an = inv_digamma(y, a, solve);
+        if (solve) a = an;
+      }
     }
-    S0a = warp_sum(S0a);
-    S1a = warp_sum(S1a);
-    SLa = warp_sum(SLa);
-    S0b = warp_sum(S0b);
-    S1b = warp_sum(S1b);
-    SLb = warp_sum(SLb);
-    ll = warp_sum(L) / s0;
-    w = fmin(fmax(S0a / (S0a + S0b), 1e-4), 1 - 1e-4);
-    for (int j = 0; j < 3; ++j) {
-      th = (S1a + S1b) / (a1 * S0a + a2 * S0b);
-      if (S0a > 0) a1 = inv_digamma(SLa / S0a - log(th));
-      if (S0b > 0) a2 = inv_digamma(SLb / S0b - log(th));
+    const double oa = __shfl_xor_sync(kAll, a, 1);
+    if (pair >= 0 && !(lane & 1)) {
+      float* o = out + pair * 5;
+      const bool swap = a > oa;  // order the components
+      const float nan = __int_as_float(0x7fc00000);
+      o[0] = live ? (float)(swap ? 1 - w : w) : nan;
+      o[1] = live ? (float)(swap ? oa : a) : nan;
+      o[2] = live ? (float)(swap ? a : oa) : nan;
+      o[3] = live ? (float)th : nan;
+      o[4] = live ? (float)ll : nan;
     }
-  }
-  if (a1 > a2) {  // order the components
-    const double x = a1;
-    a1 = a2;
-    a2 = x;
-    w = 1 - w;
-  }
-  if (lane == 0) {
-    o[0] = (float)w;
-    o[1] = (float)a1;
-    o[2] = (float)a2;
-    o[3] = (float)th;
-    o[4] = (float)ll;
+    __syncwarp();
   }
 }
 
@@ -1322,10 +1452,13 @@ extern "C" pp_status pp_gamma_mixture_fit(const double* d_hist, int64_t n, int32
   if (n < 0 || bins <= 0 || !(bin_width > 0.f) || iters < 1 || (n > 0 && (!d_hist || !d_tshift || !d_out)))
     return PP_ERR_ARG;
   if (n == 0) return PP_OK;
-  const int64_t threads = n * 32;
-  const int grid = (int)((threads + 255) / 256);
-  mlp::gamma_fit_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(d_hist, n, bins, t0, bin_width,
-                                                                              d_tshift, d_out, iters);
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) ||
+      cudaFuncSetAttribute(mlp::gamma_fit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp::kMixSmem))
+    return PP_ERR_CUDA;
+  const int grid = (int)std::min<int64_t>(n, sms);
+  mlp::gamma_fit_kernel<<<grid, mlp::kMixWarps * 32, mlp::kMixSmem, static_cast<cudaStream_t>(stream)>>>(
+      d_hist, n, bins, t0, bin_width, d_tshift, d_out, iters);
   pp::count_launches(1);
   return cudaGetLastError() ? PP_ERR_CUDA : PP_OK;
 }
