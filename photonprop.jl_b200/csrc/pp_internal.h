@@ -46,9 +46,9 @@ void count_launches(uint64_t n);
 // programmatic dependent): it waits itself, by griddepcontrol.wait, before it
 // reads what that kernel writes.
 template <typename... P, typename... A>
-cudaError_t launch_dependent(void (*fn)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
+cudaError_t launch_dependent(void (*fn)(P...), dim3 grid, int block, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
