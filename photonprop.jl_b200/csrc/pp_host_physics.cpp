@@ -79,6 +79,17 @@ void gauss_legendre(int n, std::vector<double>& x, std::vector<double>& w) {
   }
 }
 
+// The 50-point rule, computed once per process (38 us; a light-yield call uses
+// it twice).
+struct Rule50 {
+  std::vector<double> x, w;
+  Rule50() { gauss_legendre(50, x, w); }
+};
+const Rule50& rule50() {
+  static const Rule50 r;
+  return r;
+}
+
 // Photons per cm in [a, b]: GL-50 quadrature of the Frank-Tamm formula
 // 2 pi alpha / wl^2 (1 - 1/n^2) (frank_tamm / frank_tamm_norm,
 // src/spectrum.jl:32-45; integrate_gauss_quad, src/utils.jl:63-78).
@@ -101,19 +112,14 @@ double frank_tamm_norm(const pp_medium_desc* m, double a, double b, const std::v
 
 namespace pp {
 
-void gl_nodes(int n, double* x, double* w) {
-  std::vector<double> xv, wv;
-  gauss_legendre(n, xv, wv);
-  for (int i = 0; i < n; ++i) {
-    x[i] = xv[i];
-    w[i] = wv[i];
-  }
+void gl50_nodes(double* x, double* w) {
+  const Rule50& r = rule50();
+  std::copy(r.x.begin(), r.x.end(), x);
+  std::copy(r.w.begin(), r.w.end(), w);
 }
 
 double frank_tamm_norm_cm(const pp_medium_desc* m, double wl_min, double wl_max) {
-  std::vector<double> x, w;
-  gauss_legendre(50, x, w);
-  return frank_tamm_norm(m, wl_min, wl_max, x, w);
+  return frank_tamm_norm(m, wl_min, wl_max, rule50().x, rule50().w);
 }
 
 void medium_coeffs(const pp_medium_desc* m, double out[11]) {

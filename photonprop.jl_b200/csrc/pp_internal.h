@@ -150,7 +150,7 @@ cudaError_t launch_fit_columns(const FitConsts& K, const void* tables, int64_t n
                                double* fits, int sm_count, cudaStream_t s);
 
 // host physics (pp_host_physics.cpp)
-void gl_nodes(int n, double* x, double* w);  // Gauss-Legendre nodes and weights on [-1, 1]
+void gl50_nodes(double* x, double* w);  // the 50-point Gauss-Legendre nodes and weights on [-1, 1]
 double frank_tamm_norm_cm(const pp_medium_desc* m, double wl_min, double wl_max);  // photons per cm
 void medium_coeffs(const pp_medium_desc* m, double out[11]);
 void default_abs_table(double* wl, double* len, int* n);
