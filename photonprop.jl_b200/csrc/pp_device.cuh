@@ -590,7 +590,9 @@ __device__ __forceinline__ bool emit_event(const DevTables& T, const RunParams& 
 // is read).  `more` says whether the photon has another step coming, which
 // for a photon that ends out of reach is the step that would end it: the
 // photon steps of a run are the emissions (each has a first step) plus these.
-template <int MODE>
+// kLast: the photon's last step (number max_steps), which can hit but is not
+// followed by another, so that a compat-mode photon neither moves on nor turns.
+template <int MODE, bool kLast = false>
 __device__ __forceinline__ bool step_event(const RunParams& R, const PairCtx& c, Photon& s, bool& hit, bool& more) {
   uint32_t w0 = s.sc0, w1 = s.sc1 + s.ctr3;
   philox2x32_10(w0, w1, kStepKey);
@@ -607,6 +609,15 @@ __device__ __forceinline__ bool step_event(const RunParams& R, const PairCtx& c,
   s.ctr3 += 1u << 8;
   if (MODE == kCompat) {
     hit = geo;
+    more = !geo && s.ctr3 < R.ctr_limit;  // at most max_steps steps
+    if (kLast) {
+      const float2 pxy = __ffma2_rn(make_float2(dd, dd), make_float2(s.dx, s.dy), make_float2(s.px, s.py));
+      s.px = pxy.x;
+      s.py = pxy.y;
+      s.pz = fmaf(dd, s.dz, s.pz);
+      s.path += dd;
+      return more;
+    }
     const bool move = !(b >= 0.f);  // the line meets the sphere outside this step: no move (reference)
     const float len = hit ? dd : (move ? step : 0.f);
     const float2 pxy = __ffma2_rn(make_float2(len, len), make_float2(s.dx, s.dy), make_float2(s.px, s.py));
@@ -618,7 +629,6 @@ __device__ __forceinline__ bool step_event(const RunParams& R, const PairCtx& c,
     s.dx = move ? rx : s.dx;
     s.dy = move ? ry : s.dy;
     s.dz = move ? rz : s.dz;
-    more = !geo && s.ctr3 < R.ctr_limit;  // at most max_steps steps
     return more;
   } else {
     hit = geo && dd <= s.path;  // arrives inside the time window
@@ -764,6 +774,51 @@ __device__ __forceinline__ void flush_warp_stats(double* stats, WarpStats* ws) {
   for (int k = 0; k < 6; ++k) ws->v[k] = 0.0;
 }
 
+// The six sums of a converged warp's hits (valid lanes, pairs as they come):
+// those of the cached pair are added over the warp and kept by one lane, the
+// others go to the global sums.  (As shared-memory atomics, 32 lanes on six
+// addresses took 163 compare-and-swap rounds.)
+__device__ __forceinline__ void add_warp_stats(const RunParams& R, WarpStats* ws, bool valid, int pair,
+                                               const HitValues& h) {
+  const double w = (double)h.weight, t = (double)h.time;
+  double v[6] = {1.0, w, w * w, w * t, w * t * t, w * (double)logf(h.time)};
+  const bool cached = valid && pair == ws->pair;
+  if (valid && !cached) {
+    double* st = R.stats + (int64_t)pair * PP_STATS;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) atomicAdd(st + k, v[k]);
+  }
+  const unsigned lane = threadIdx.x & 31u;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) v[k] = cached ? v[k] : 0.0;
+  // lanes with an even index take the first three sums, the others the rest
+  double u[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double give = (lane & 1u) ? v[k] : v[k + 3];
+    u[k] = ((lane & 1u) ? v[k + 3] : v[k]) + __shfl_xor_sync(kFull, give, 1);
+  }
+#pragma unroll
+  for (int o = 2; o < 32; o <<= 1)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) u[k] += __shfl_xor_sync(kFull, u[k], o);
+  if (lane < 2u)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) ws->v[3 * lane + k] += u[k];
+}
+
+// Histogram and record of one lane's hit, its sums taken already.
+__device__ __forceinline__ void store_hit(const RunParams& R, const PairCtx& c, const Photon& s, const HitValues& h) {
+  histogram_hit(R, h, c.index);
+  const unsigned m = __activemask();
+  const int leader = __ffs(m) - 1;
+  const unsigned lane = threadIdx.x & 31u;
+  unsigned long long base = 0;
+  if ((int)lane == leader) base = atomicAdd(R.counters + 0, (unsigned long long)__popc(m));
+  base = __shfl_sync(m, base, leader);
+  write_hit(R, c, s, h, base + __popc(m & ((1u << lane) - 1u)));
+}
+
 // record_hit with the warp's statistics cache: lanes whose pair is the
 // cached one add to it (shared-memory atomics), others to the global sums.
 __device__ __forceinline__ void record_hit_cached(const RunParams& R, WarpStats* ws, const PairCtx& c,
@@ -777,14 +832,7 @@ __device__ __forceinline__ void record_hit_cached(const RunParams& R, WarpStats*
   atomicAdd(st + 3, w * t);
   atomicAdd(st + 4, w * t * t);
   atomicAdd(st + 5, w * (double)logf(h.time));
-  histogram_hit(R, h, c.index);
-  const unsigned m = __activemask();
-  const int leader = __ffs(m) - 1;
-  const unsigned lane = threadIdx.x & 31u;
-  unsigned long long base = 0;
-  if ((int)lane == leader) base = atomicAdd(R.counters + 0, (unsigned long long)__popc(m));
-  base = __shfl_sync(m, base, leader);
-  write_hit(R, c, s, h, base + __popc(m & ((1u << lane) - 1u)));
+  store_hit(R, c, s, h);
 }
 
 }  // namespace ppd

@@ -44,9 +44,12 @@ namespace ppd {
 // photons): 3.00e9 -> 2.36e9 warp instructions, 3.47 -> 2.85 ms, by testing
 // the reach where a photon stops (in_reach), one emission pass per pair with
 // its record by broadcast, and separate loops for the full warp and for the
-// last photons; 4096 mixed pairs (5.75e9 photons): 171 -> 139 ms; compat
-// mode in lockstep, 100 distances of 2e7 photons with their fits: 175 -> 130
-// ms.  Measured and not kept: the first one or two steps inside the emission
+// last photons; 4096 mixed pairs (5.75e9 photons): 171 -> 139 ms.  Compat mode
+// (100 distances, 2e9 photons): 139.4 -> 90.1 ms, 124 warp instructions per
+// step with the emission's tenth and the hits; the last step leaves out the
+// move and turn that nothing follows, steps are counted by what hits leave
+// out, a batch of hits adds its sums over the warp.  Measured and not kept:
+// the first one or two steps of physical mode inside the emission
 // pass (fewer loop iterations, but 180 bytes spilled at 64 registers: 3.26 ms).
 constexpr int kStage = 64;  // >= 2 * 32 - 1 staged emissions per warp (power of two)
 
@@ -69,6 +72,7 @@ struct __align__(16) WarpArea {
   unsigned long long run_at, run_end;  // the granules of the run that follow in other pairs
   unsigned left;                       // the pair's photons left in the run
   int pair;
+  unsigned long long not_made;  // compat: steps that hits left out
   WarpStats stats;
 };
 static_assert(sizeof(pp_pair) == 5 * sizeof(float4), "the record is copied as 16-byte words");
@@ -84,6 +88,7 @@ struct StagedHit {
   float px, py, pz, dx, dy, dz, path;
   uint32_t id_lo, id_hi;
   int32_t pair;
+  int32_t left;  // steps that the hit leaves out
 };
 
 // Register budget: 64 per thread (1024 threads per SM) for the basic
@@ -104,6 +109,7 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
     for (int k = 0; k < 6; ++k) wa->stats.v[k] = 0.0;
     wa->left = 0;
     wa->pair = 0;
+    wa->not_made = 0;
     wa->run_at = wa->run_end = 0;
   }
   __syncthreads();
@@ -116,57 +122,61 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
   // records staged hits 0..n-1 (n warp-uniform), one per lane
   auto record_staged = [&](unsigned n) {
     __syncwarp();
-    if (lane < n) {
-      const StagedHit& g = hst[lane];
-      Photon p;
-      p.px = g.px;
-      p.py = g.py;
-      p.pz = g.pz;
-      p.dx = g.dx;
-      p.dy = g.dy;
-      p.dz = g.dz;
-      p.path = g.path;
-      p.neg_ln2_len = 0.f;
-      p.id_lo = g.id_lo;
-      p.ctr3 = g.id_hi;  // block 0: the index's top bits only
-      p.sc0 = p.sc1 = 0u;
-      const PairCtx pc{0.f, g.pair};
-      const HitValues h = hit_values<MODE, EM>(T, R, R.pairs + g.pair, p);
-      record_hit_cached(R, ws, pc, p, h);
-    }
+    const bool valid = lane < n;
+    const StagedHit& g = hst[valid ? lane : 0u];
+    Photon p;
+    p.px = g.px;
+    p.py = g.py;
+    p.pz = g.pz;
+    p.dx = g.dx;
+    p.dy = g.dy;
+    p.dz = g.dz;
+    p.path = g.path;
+    p.neg_ln2_len = 0.f;
+    p.id_lo = g.id_lo;
+    p.ctr3 = g.id_hi;  // block 0: the index's top bits only
+    p.sc0 = p.sc1 = 0u;
+    const PairCtx pc{0.f, g.pair};
+    const HitValues h = hit_values<MODE, EM>(T, R, R.pairs + g.pair, p);
+    add_warp_stats(R, ws, valid, g.pair, h);
+    const unsigned less = __reduce_add_sync(kFull, valid ? (unsigned)g.left : 0u);
+    if (lane == 0) wa->not_made += less;
+    if (valid) store_hit(R, pc, p, h);
     __syncwarp();
   };
   // takes the hits of a step (all lanes call)
-  auto take_hits = [&](bool hit, const Photon& p, const PairCtx& c) {
+  auto take_hits = [&](bool hit, const Photon& p, const PairCtx& c, int left) -> bool {
     if (MODE == kCompat) {
       const unsigned hm = __ballot_sync(kFull, hit);
-      if (hm) {
-        const unsigned nh = __popc(hm);
-        if (h_count + nh > kHitStage) {  // no room: record what is staged first
-          record_staged(h_count);
-          h_count = 0;
-        }
-        if (hit) {
-          StagedHit& g = hst[h_count + __popc(hm & lt_mask)];
-          g.px = p.px;
-          g.py = p.py;
-          g.pz = p.pz;
-          g.dx = p.dx;
-          g.dy = p.dy;
-          g.dz = p.dz;
-          g.path = p.path;
-          g.id_lo = p.id_lo;
-          g.id_hi = p.ctr3 & 0xFFu;
-          g.pair = c.index;
-        }
-        h_count += nh;
+      if (!hm) return false;
+      const unsigned nh = __popc(hm);
+      if (h_count + nh > kHitStage) {  // no room: record what is staged first
+        record_staged(h_count);
+        h_count = 0;
       }
-    } else if (__any_sync(kFull, hit)) {
       if (hit) {
-        const HitValues h = hit_values<MODE, EM>(T, R, R.pairs + c.index, p);
-        record_hit_cached(R, ws, c, p, h);
+        StagedHit& g = hst[h_count + __popc(hm & lt_mask)];
+        g.px = p.px;
+        g.py = p.py;
+        g.pz = p.pz;
+        g.dx = p.dx;
+        g.dy = p.dy;
+        g.dz = p.dz;
+        g.path = p.path;
+        g.id_lo = p.id_lo;
+        g.id_hi = p.ctr3 & 0xFFu;
+        g.pair = c.index;
+        g.left = left;
       }
+      h_count += nh;
+      return true;
     }
+    if (!__any_sync(kFull, hit)) return false;
+    if (hit) {
+      const HitValues h = hit_values<MODE, EM>(T, R, R.pairs + c.index, p);
+      record_hit_cached(R, ws, c, p, h);
+    }
+    return true;
   };
   // the next pair of the warp's run, or of its next run, with its record and
   // statistics cache; false when the queue is exhausted.  A run is half the
@@ -214,7 +224,7 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
   };
   // emits the pair's next photons, one per lane (lanes past its last photon
   // emit as well, and drop it); returns whether the lane has one that is in reach
-  unsigned steps = 0;  // beyond the photons' first ones, which the set-up kernel has counted
+  unsigned steps = 0;  // beyond those that the set-up kernel has counted (physical mode)
   auto emit = [&](Photon& e, PairCtx& c) {
     const unsigned left = wa->left, n = min(32u, left);
     const uint64_t base = wa->base;
@@ -234,15 +244,17 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
       if (wa->left == 0u && !fetch()) break;
       Photon s;
       PairCtx c;
-      bool alive = emit(s, c);
-      do {
-        bool hit, more;
+      bool alive = emit(s, c), hit, more;
+      for (int left = R.max_steps - 1; left > 0; --left) {
         step_event<MODE>(R, c, s, hit, more);
-        more = more && alive;
-        take_hits(hit && alive, s, c);
-        steps += more ? 1u : 0u;
-        alive = more;
-      } while (__any_sync(kFull, alive));
+        hit = hit && alive;
+        if (take_hits(hit, s, c, left)) {
+          alive = alive && !hit;
+          if (!__any_sync(kFull, alive)) break;
+        }
+      }
+      step_event<MODE, true>(R, c, s, hit, more);
+      take_hits(hit && alive, s, c, 0);
     }
   } else {
     // warp-uniform state of the ring, and the lane's photon and pair (radius
@@ -311,7 +323,7 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
       bool hit, more;
       alive = step_event<MODE>(R, c, s, hit, more);
       steps += more ? 1u : 0u;
-      take_hits(hit, s, c);
+      take_hits(hit, s, c, 0);
     }
     // The ring's last photons, then ever fewer lanes.
     for (;;) {
@@ -327,7 +339,7 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
       bool hit = false, more = false;
       if (alive) alive = step_event<MODE>(R, c, s, hit, more);
       steps += more ? 1u : 0u;
-      take_hits(hit, s, c);
+      take_hits(hit, s, c, 0);
     }
   }
   if (MODE == kCompat && h_count > 0u) record_staged(h_count);
@@ -335,8 +347,12 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
   if (lane == 0) flush_warp_stats(R.stats, ws);
   // photon-step count for the roofline
   unsigned long long st = steps;
+  if (MODE == kCompat) {
+    st = 0ull - wa->not_made;
+  } else {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) st += __shfl_xor_sync(kFull, st, o);
+    for (int o = 16; o > 0; o >>= 1) st += __shfl_xor_sync(kFull, st, o);
+  }
   if (lane == 0) atomicAdd(R.counters + 1, st);
 }
 
@@ -462,16 +478,17 @@ __global__ void __launch_bounds__(1024) fill_kernel(const pp_pair* __restrict__ 
 
 // The work queue of a launch.  Block 0 resets the queue cursor and the
 // counters and writes the offsets: offsets[p] = granules (32 photons) of pairs
-// 0..p-1, offsets[n] all of them; counters[1] starts as the photons' first
-// steps (one each), to which the batched kernel adds the others.  offsets ==
-// NULL (the one-pair kernel, which counts all its steps): no queue.  Further
-// blocks, if any, fill the outputs.
+// 0..p-1, offsets[n] all of them; counters[1] starts as photon_steps per
+// photon: physical mode the first one, to which the batched kernel adds the
+// others, compat mode max_steps, from which it takes what hits leave out.
+// offsets == NULL (the one-pair kernel, which counts all its steps): no queue.
+// Further blocks, if any, fill the outputs.
 __global__ void __launch_bounds__(1024) setup_kernel(const pp_pair* __restrict__ pairs, int64_t n,
                                                      unsigned long long* __restrict__ offsets,
                                                      unsigned long long* __restrict__ queue,
                                                      unsigned long long* __restrict__ counters,
                                                      double* __restrict__ stats, double* __restrict__ hist,
-                                                     int64_t hist_len) {
+                                                     int64_t hist_len, unsigned photon_steps) {
   // the batched kernel may start (its blocks wait for this grid to end
   // before they read what it writes)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -537,7 +554,7 @@ __global__ void __launch_bounds__(1024) setup_kernel(const pp_pair* __restrict__
       queue[0] = 0ull;
     }
     counters[0] = 0ull;
-    counters[1] = all;
+    counters[1] = all * photon_steps;
     counters[2] = 0ull;
     counters[3] = 0ull;
   }
@@ -788,9 +805,10 @@ cudaError_t launch_setup(const LaunchArgs& a, int sm_count, cudaStream_t s) {
   // the outputs have a kernel of their own, which the scan's registers do not
   // hold to one block per SM.
   const int64_t blocks = (words + 16383) / 16384;
+  const unsigned photon_steps = a.opts.mode == PP_MODE_COMPAT ? (unsigned)a.opts.max_steps : 1u;
   if (blocks <= 1) {
     ppd::setup_kernel<<<1 + (int)blocks, 1024, 0, s>>>(a.pairs, a.n_pairs, a.granule_offsets, a.queue, a.counters,
-                                                       a.stats, a.hist, hist_len);
+                                                       a.stats, a.hist, hist_len, photon_steps);
     count_launches(1);
     return cudaGetLastError();
   }
@@ -800,7 +818,7 @@ cudaError_t launch_setup(const LaunchArgs& a, int sm_count, cudaStream_t s) {
   const cudaError_t e = cudaGetLastError();
   if (e) return e;
   return launch_dependent(ppd::setup_kernel, 1, 1024, 0, s, a.pairs, a.n_pairs, a.granule_offsets, a.queue, a.counters,
-                          (double*)nullptr, (double*)nullptr, (int64_t)0);
+                          (double*)nullptr, (double*)nullptr, (int64_t)0, photon_steps);
 }
 
 namespace {
