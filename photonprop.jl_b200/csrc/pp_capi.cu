@@ -982,7 +982,8 @@ pp_status pp_propagate_fit(pp_ctx* c, const pp_pair* pairs, int64_t n_pairs, con
                                          static_cast<const unsigned long long*>(c->counters.p),
                                          static_cast<unsigned long long*>(c->fit_counts.p),
                                          static_cast<pp::FitRec*>(c->fit_rec.p),
-                                         static_cast<const float2*>(c->fit_cs.p), n_angles, d_mom, c->sm_count, s)))
+                                         static_cast<const float2*>(c->fit_cs.p), n_angles, d_mom, c->sm_count, s,
+                                         static_cast<const double*>(c->stats.p), start, end)))
       return c->cuda_fail(e, "fit moments");
     total += (int64_t)cnt[0];
     start = end;

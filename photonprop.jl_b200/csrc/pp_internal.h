@@ -136,11 +136,14 @@ struct FitRec {  // 32 bytes, one per hit
 static_assert(sizeof(FitRec) == 32, "FitRec is moved as two 16-byte words");
 void fill_fit_consts(FitConsts* K, double n800_phase, double n800_group);
 // Adds the moments of the stored hits (their pair fields index `pairs`) to
-// moments [n_pairs x n_angles x 4]; the caller zeroes moments first.
+// moments [n_pairs x n_angles x 4]; the caller zeroes moments first.  stats
+// (may be NULL): the statistics of the propagation of pairs [lo, hi) that
+// stored all its hits there, whose hit counts are then not counted again.
 cudaError_t launch_fit_moments_hits(const FitConsts& K, const void* tables, const pp_pair* pairs, int64_t n_pairs,
                                     int mode, const pp_hit* hits, unsigned long long cap,
                                     const unsigned long long* counters, unsigned long long* counts, FitRec* rec,
-                                    const float2* cs, int n_angles, double* moments, int sm_count, cudaStream_t s);
+                                    const float2* cs, int n_angles, double* moments, int sm_count, cudaStream_t s,
+                                    const double* stats = nullptr, int64_t lo = 0, int64_t hi = 0);
 // Gamma fits and detection fractions of every (pair, angle) from the moments.
 cudaError_t launch_fit_gamma(const double* moments, int64_t n_pairs, int n_angles, const pp_pair* pairs,
                              int64_t n_gen, double* fits, cudaStream_t s);

@@ -7,26 +7,6 @@
 
 namespace ppsf {
 
-__device__ __forceinline__ double digamma_d(double x) {
-  double r = 0.0;
-  while (x < 6.0) {
-    r -= 1.0 / x;
-    x += 1.0;
-  }
-  const double f = 1.0 / (x * x);
-  return r + log(x) - 0.5 / x - f * (1.0 / 12 - f * (1.0 / 120 - f * (1.0 / 252 - f * (1.0 / 240 - f / 132))));
-}
-
-__device__ __forceinline__ double trigamma_d(double x) {
-  double r = 0.0;
-  while (x < 6.0) {
-    r += 1.0 / (x * x);
-    x += 1.0;
-  }
-  const double f = 1.0 / (x * x);
-  return r + 1.0 / x + 0.5 * f + (1.0 / x) * f * (1.0 / 6 - f * (1.0 / 30 - f * (1.0 / 42 - f / 30)));
-}
-
 // psi(x) and psi'(x) together, x > 0, with one reciprocal for the recurrence:
 // below 6 the argument is shifted by 6, whose six terms pair up with
 // q = x (x + 5), q + 4 = (x + 1)(x + 4), q + 6 = (x + 2)(x + 3):
