@@ -124,6 +124,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
   return false;
 }
 
+// Bulk copy of global to shared memory, completing on the mbarrier (its one arrival).
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint32_t mbar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(mbar)
+               : "memory");
+}
+
 // 32 FP32 accumulator columns [col, col+32) of this thread's row.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   uint32_t r[32];
@@ -313,16 +322,17 @@ __global__ void __launch_bounds__(INFER_THREADS, 1) infer_kernel(DevParams P, co
   float* b4 = reinterpret_cast<float*>(acts + kGroups * TILE * H);
   float* nrm = b4 + 8;
   uint64_t* mbars = reinterpret_cast<uint64_t*>(nrm + 24);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(mbars + kGroups);
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(mbars + kGroups + 2);
 
   const int t = threadIdx.x;
   const int g = t >> 7, gt = t & (THREADS - 1);  // group, thread (= row) within the group
-  load_tile(w2, P.w2h);
-  load_tile(w3, P.w3h);
-  {
-    const int4* s1 = reinterpret_cast<const int4*>(P.w1tc);
-    int4* d1 = reinterpret_cast<int4*>(w1t);
-    for (int i = t; i < 4 * H * 16 * 2 / 16; i += INFER_THREADS) d1[i] = s1[i];  // W1, W4, b2, b3 tiles
+  // the weight tiles (W1, W4, b2, b3 contiguous, then W2 and W3), as bulk
+  // copies that the first tile's layers wait for
+  const uint32_t mb_narrow = smem_u32(mbars + kGroups), mb_wide = smem_u32(mbars + kGroups + 1);
+  if (t == 0) {
+    for (int i = 0; i < kGroups + 2; ++i) mbar_init(smem_u32(mbars + i));
+    bulk_load(w1t, P.w1tc, 4 * H * 16 * 2, mb_narrow);
+    bulk_load(w2, P.w2h, 2 * TILE_BYTES, mb_wide);
   }
   for (int i = t; i < TILE * 16 / 8; i += INFER_THREADS) {  // the ones tile, 8 columns per 16-byte word
     const int row = i >> 1, k8 = i & 1;
@@ -333,7 +343,6 @@ __global__ void __launch_bounds__(INFER_THREADS, 1) infer_kernel(DevParams P, co
   if (t < OUT) b4[t] = P.p[OFF_B4 + t];
   if (t < 18) nrm[t] = P.norm[t];
   if (t < IN) nrm[18 + t] = 1.f / P.norm[4 + t];  // feature scales as reciprocals: no division per row
-  if (t < kGroups) mbar_init(smem_u32(mbars + t));
   if ((t >> 5) == 0) {  // all 512 columns: 128 per group
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tslot)));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -349,16 +358,21 @@ __global__ void __launch_bounds__(INFER_THREADS, 1) infer_kernel(DevParams P, co
   uint32_t parity = 0;
   bool ok = true;
 
-  const int64_t tile_step = (int64_t)gridDim.x * kGroups;
+  // tiles go to the blocks first and to their groups second, so that a few
+  // thousand queries have an SM per tile (3001 queries: four tiles on each of
+  // six SMs 16.6 us, one tile on each of 24 SMs 10.2 us per call)
+  const int64_t tile_step = (int64_t)gridDim.x * kGroups, tile0 = blockIdx.x + (int64_t)g * gridDim.x;
   // the row's features, loaded one tile ahead so that the global loads
   // overlap the previous tile's layers
   float xr[IN];
   {
-    const int64_t row0 = ((int64_t)blockIdx.x * kGroups + g) * TILE + gt;
+    const int64_t row0 = tile0 * TILE + gt;
 #pragma unroll
     for (int j = 0; j < IN; ++j) xr[j] = row0 < n ? x[row0 * IN + j] : nrm[j];
   }
-  for (int64_t tile = (int64_t)blockIdx.x * kGroups + g; ok && tile * TILE < n; tile += tile_step) {
+  if (tile0 * TILE < n) ok = group_all(g, mbar_wait(mb_narrow, 0));
+  bool wide = false;  // W2 and W3 are here
+  for (int64_t tile = tile0; ok && tile * TILE < n; tile += tile_step) {
     const int64_t row = tile * TILE + gt;
     const bool valid = row < n;
     float xn[8];
@@ -401,6 +415,11 @@ __global__ void __launch_bounds__(INFER_THREADS, 1) infer_kernel(DevParams P, co
       for (int q = 0; q < 4; ++q) store8(act, gt, c * 4 + q, v + q * 8);
     }
     // layer 2
+    if (!wide) {
+      ok = group_all(g, mbar_wait(mb_wide, 0));
+      if (!ok) break;
+      wide = true;
+    }
     ok = group_layer(2, act, w2, tmem, mb, parity, g, gt, ones, b2t);
     if (!ok) break;
     for (int c = 0; c < 4; ++c) {
@@ -448,7 +467,11 @@ __global__ void __launch_bounds__(INFER_THREADS, 1) infer_kernel(DevParams P, co
       }
     }
   }
-  if (!ok && gt == 0) atomicExch(P.error, 1);
+  if (!ok && gt == 0) {
+    atomicExch(P.error, 1);
+    mbar_wait(mb_narrow, 0);  // the block's copies in flight
+    mbar_wait(mb_wide, 0);
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1171,7 +1194,7 @@ __global__ void __launch_bounds__(kMixWarps * 32, 1) gamma_fit_kernel(const doub
   }
 }
 
-constexpr size_t kInferSmem = (2 + kGroups) * TILE_BYTES + 5 * H * 16 * 2 + (8 + 24) * 4 + 8 * kGroups + 16;
+constexpr size_t kInferSmem = (2 + kGroups) * TILE_BYTES + 5 * H * 16 * 2 + (8 + 24) * 4 + 8 * (kGroups + 2) + 16;
 constexpr size_t kTrainSmem = 6 * TILE_BYTES + (H * IN + H * 8 + TILE * 8 + TILE * IN + 3 * H) * 4 + 16;
 constexpr size_t kTestSmem = 2 * TILE_BYTES + 32;
 
@@ -1364,7 +1387,7 @@ pp_status pp_mlp_forward(pp_mlp* m, const float* d_x, float* d_out, int64_t n, i
   std::lock_guard<std::mutex> lk(m->mu);
   Guard g(m->device);
   const int64_t tiles = (n + mlp::TILE - 1) / mlp::TILE;
-  const int grid = (int)std::min<int64_t>((tiles + mlp::kGroups - 1) / mlp::kGroups, (int64_t)m->sm_count);
+  const int grid = (int)std::min<int64_t>(tiles, (int64_t)m->sm_count);
   mlp::infer_kernel<<<grid, mlp::INFER_THREADS, mlp::kInferSmem, static_cast<cudaStream_t>(stream)>>>(
       dev_params(m), d_x, d_out, n, physical);
   pp::count_launches(1);

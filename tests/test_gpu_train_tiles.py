@@ -57,3 +57,21 @@ def test_empty_mask_moves_nothing():
     loss, g = net.train_step(torch.ones((200, 4), device="cuda"), z + 1.0, z, 200, 0.0, want_grads=True)
     assert loss == 0.0 and not np.any(g)
     net.close()
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 3001, 148 * 128, 148 * 128 + 1, 80_000])
+def test_a_query_is_answered_alike_in_any_batch(n):
+    """Tiles over blocks and groups: the rows of a batch of n are those of a batch of 100,001, bit for bit."""
+    import torch
+    from photonprop_b200 import surrogate as sg
+    net = sg.MLP(0, 8)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn((100_001, 4), generator=g, device="cuda")
+    a, b = torch.zeros((5, 100_001), device="cuda"), torch.full((5, n), 7.0, device="cuda")
+    net.forward(x, a, 100_001)
+    net.forward(x[:n].contiguous(), b, n)
+    torch.cuda.synchronize()
+    assert torch.equal(a[:, :n], b)
+    want, _ = omlp.forward(net.get_params().astype(np.float64), x[-5:].cpu().numpy().astype(np.float64))
+    np.testing.assert_allclose(a[:, -5:].cpu().numpy().T, want, rtol=2e-2, atol=2e-2)
+    net.close()
