@@ -30,8 +30,13 @@
 #include <cstdint>
 
 #include "pp_internal.h"
+#include "pp_special.cuh"
 
 namespace {
+
+using ppsf::WarpTables;
+using ppsf::exp_tab;
+using ppsf::log_tab;
 
 constexpr int kThreads = 128, kWarps = kThreads / 32;
 constexpr int kTile = 512;           // sources per shared-memory tile
@@ -63,86 +68,6 @@ __device__ __forceinline__ void lse_add(double v, double& m, double& s) {
   } else {
     s += exp(v - m);
   }
-}
-
-// Table-driven exponential and logarithm (P. T. P. Tang, ACM TOMS 15 (1989)
-// 144 and 16 (1990) 378): the argument is reduced to 1/32 of an octave, the
-// remainder's Taylor series needs few terms, and a warp's 32 lanes hold the
-// table, one entry each, which a lookup takes by shuffle (all lanes take part).
-// Against the FP64 values: exp within 1 ulp, log within 2e-16 + 1 ulp.
-struct WarpTables {
-  double exp2_at;         // 2^(lane / 32)
-  double inv_at, log_at;  // 1 / c, rounded to FP32, and ln c, for c at the middle of [1 + lane/32, 1 + (lane + 1)/32)
-  // the constants, held in registers: as literals or from constant memory
-  // each costs one or two instructions per use
-  double inv_ln2_32, magic, ln2_32_hi, ln2_32_lo;  // 32 / ln 2; 1.5 * 2^52; -ln 2 / 32 as 37 leading bits and the rest
-  double e3, e4, e5, e6;                           // 1 / n!
-  double bias, ln2;                                // 2^52 + 1023
-  double l3, l4, l5, l6, l7, l8;                   // -(-1)^n / n
-};
-__device__ __forceinline__ double in_register(double v) {
-  double r;
-  asm volatile("mov.f64 %0, %1;" : "=d"(r) : "d"(v));
-  return r;
-}
-__device__ __forceinline__ WarpTables warp_tables() {
-  const double l = (double)(threadIdx.x & 31);
-  WarpTables t;
-  t.exp2_at = exp2(l / 32.0);
-  t.inv_at = (double)(float)(1.0 / (1.0 + (l + 0.5) / 32.0));
-  t.log_at = -log(t.inv_at);
-  t.inv_ln2_32 = in_register(32.0 / 0.69314718055994530942);
-  t.magic = in_register(6755399441055744.0);
-  t.ln2_32_hi = in_register(-0x1.62e42fefap-6);
-  t.ln2_32_lo = in_register(-0x1.cf79abc9e3b39p-45);
-  t.e3 = in_register(1.0 / 6);
-  t.e4 = in_register(1.0 / 24);
-  t.e5 = in_register(1.0 / 120);
-  t.e6 = in_register(1.0 / 720);
-  t.bias = in_register(4503599627371519.0);
-  t.ln2 = in_register(0.69314718055994530942);
-  t.l3 = in_register(1.0 / 3);
-  t.l4 = in_register(-1.0 / 4);
-  t.l5 = in_register(1.0 / 5);
-  t.l6 = in_register(-1.0 / 6);
-  t.l7 = in_register(1.0 / 7);
-  t.l8 = in_register(-1.0 / 8);
-  return t;
-}
-// e^v for -708 <= v <= 708; beyond, the value at that end (an argument that is
-// not a number gives one of the two).
-__device__ __forceinline__ double exp_tab(double v, const WarpTables& T) {
-  constexpr unsigned kLow = 0xC0862000u;  // high word of -708
-  constexpr int kHigh = 0x40862000;       // high word of 708
-  const int hi = min((int)min((unsigned)__double2hiint(v), kLow), kHigh);
-  v = __hiloint2double(hi, __double2loint(v));
-  const double t = fma(v, T.inv_ln2_32, T.magic);  // rounded to an integer, in the low word
-  const int n = __double2loint(t);
-  const double k = t - T.magic;
-  const double r = fma(k, T.ln2_32_lo, fma(k, T.ln2_32_hi, v));
-  double q = fma(r, T.e6, T.e5);
-  q = fma(r, q, T.e4);
-  q = fma(r, q, T.e3);
-  q = fma(r, q, 0.5);
-  const double p = fma(r * r, q, r);
-  const double at = __shfl_sync(kAll, T.exp2_at, n);  // lane n mod 32
-  const double e = fma(at, p, at);
-  return __hiloint2double(__double2hiint(e) + ((n >> 5) << 20), __double2loint(e));
-}
-// ln y for normal y > 0 (anything else gives some number).
-__device__ __forceinline__ double log_tab(double y, const WarpTables& T) {
-  const int hi = __double2hiint(y);
-  const double m = __hiloint2double((hi & 0x000FFFFF) | 0x3FF00000, __double2loint(y));
-  const int at = hi >> 15;  // lane: the mantissa's leading five bits
-  const double k = __hiloint2double(0x43300000, hi >> 20) - T.bias;  // 2^52 + biased exponent, less 2^52 + 1023
-  const double r = fma(m, __shfl_sync(kAll, T.inv_at, at), -1.0);  // |r| <= 1/63: the series' ninth term is below 1e-17
-  double q = fma(r, T.l8, T.l7);
-  q = fma(r, q, T.l6);
-  q = fma(r, q, T.l5);
-  q = fma(r, q, T.l4);
-  q = fma(r, q, T.l3);
-  q = fma(r, q, -0.5);
-  return fma(k, T.ln2, __shfl_sync(kAll, T.log_at, at)) + fma(r * r, q, r);
 }
 
 // Hits per chunk, from the number of all hits: enough items for every block
@@ -233,7 +158,7 @@ __global__ void __launch_bounds__(kThreads, 6) llh_kernel(int mode, int64_t S, i
   __shared__ double red[kWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t h = blockIdx.y;
-  const WarpTables T = warp_tables();
+  const WarpTables T = ppsf::warp_tables();
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int64_t total = chunk_start[M], per = chunk_start[M + 1];
   for (int64_t g = blockIdx.x; g < total; g += gridDim.x) {

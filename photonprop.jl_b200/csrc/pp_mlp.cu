@@ -962,25 +962,30 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_test_kernel(const __nv_bfloat
 // weighted EM to each pair's arrival-time histogram, as a function of the
 // time residual t - t_shift (bins with a positive residual only; the reference
 // fits a single Gamma to the time residual, src/modelling.jl:52-79).
-// M step: theta = sum_k S1_k / sum_k a_k S0_k, then psi(a_k) =
+// M step: theta = sum of weight x time / sum_k a_k S0_k, then psi(a_k) =
 // SL_k / S0_k - ln theta solved by Newton, three times.  Output per pair: w,
 // a1 <= a2, theta, mean log-likelihood per weight; NaNs when the histogram is
 // empty.
 //
-// A warp fits up to 16 pairs together.  Their filled bins (weight, time, log
-// time) are gathered once into the warp's part of shared memory.  E step: the
-// warp walks one pair's bins after the other; the two densities share
-// t / theta, so their ratio takes one exponential, and the log-likelihood
-// one logarithm more, in the last iteration only.  M step: one lane per
-// (pair, component).  Bins that do not fit (a first pair of more than
+// A warp fits up to 16 pairs together.  Their filled bins (weight, log time)
+// are gathered once into the warp's part of shared memory.  E step: the warp
+// walks one pair's bins after the other, two per lane at a time; the two
+// densities share t / theta, so their ratio takes one exponential, and the
+// log-likelihood one logarithm more, in the last iteration only.  M step: one
+// lane per (pair, component).  Bins that do not fit (a first pair of more than
 // kMixEntries filled bins) are read from the histogram again each time.
 //
-// Bound by FP64 issue.  With one pair per warp, every lane did the same 48
-// digamma and trigamma evaluations per iteration: 20,000 pairs of 1000 bins
-// (60 iterations) took 36.1 ms, now 3.8 ms (issue 50 % of active cycles, FP64
-// pipe 35 %, 16 warps per SM).
-constexpr int kMixWarps = 16, kMixEntries = 768, kMixPairs = 16;
-constexpr size_t kMixSmem = (size_t)kMixWarps * kMixEntries * (2 * sizeof(double) + sizeof(uint16_t));
+// Bound by FP64 latency and issue.  With one pair per warp, every lane did the
+// same 48 digamma and trigamma evaluations per iteration: 20,000 pairs of 1000
+// bins (60 iterations) took 36.1 ms.  Shared M steps: 3.76 ms.  The table-driven
+// exponential and a reciprocal without branches, so that two bins overlap;
+// no sum for the times, whose total is known; Newton from the last evaluation
+// (one a solve, or none): 2.62 ms.  A pair taken only when there is room for
+// it: 2.53 ms; the histogram loaded four rows ahead: 2.33 ms (issue 55 % of
+// active cycles, FP64 pipe 36 %).  16 warps of 896 bins: 20 of 704 (96
+// registers) took 12 % longer, 24 of 592 17 %.
+constexpr int kMixWarps = 16, kMixEntries = 896, kMixPairs = 16;
+constexpr size_t kMixSmem = (size_t)kMixWarps * kMixEntries * sizeof(double2);
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -988,40 +993,58 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// a >= 1e-3 with psi(a) = y: Newton from the last solution, or, where that is
-// far off, from Minka's initial value.  psi is concave, so from the second
-// step on the iterates rise to the root; their error is squared by each step,
-// so a step of 1e-8 leaves none that FP64 holds.  All lanes of the warp call.
-__device__ double inv_digamma(double y, double a, bool active) {
-  for (int i = 0; i < 24; ++i) {
-    double f, f1;
-    ppsf::psi_both(a, f, f1);
-    double n = a - (f - y) / f1;
+// psi(a) = y, a >= 1e-3, by Newton from the last point that psi was evaluated
+// at (where its step is far off: from Minka's initial value).  psi is concave,
+// so from the second step on the iterates rise to the root; their error is
+// squared by each step, so a step of 1e-8 leaves none that FP64 holds, and a
+// right side that moved by less takes no evaluation.  All lanes of the warp call.
+struct Psi {
+  double at, f, rf1;  // psi and 1 / psi' at `at`
+  __device__ void eval(double x) {
+    double f1;
+    at = x;
+    ppsf::psi_both(x, f, f1);
+    rf1 = 1.0 / f1;
+  }
+};
+__device__ __forceinline__ double inv_digamma(double y, Psi& P, bool active) {
+#pragma unroll 1
+  for (int i = 0;; ++i) {
+    const double a = P.at;
+    double n = a - (P.f - y) * P.rf1;
     if (i == 0 && !(n > 0.5 * a && n < 2.0 * a)) n = y >= -2.22 ? exp(y) + 0.5 : -1.0 / (y + 0.5772156649015329);
     n = n < 1e-3 ? 1e-3 : n;
     const bool moving = active && fabs(n - a) > 1e-8 * a;
-    a = n;
-    if (!__any_sync(0xffffffffu, moving)) break;
+    if (i == 24 || !__any_sync(0xffffffffu, moving)) return n;
+    if (moving) P.eval(n);
   }
-  return a;
+}
+
+// 1 / s for 1 <= s <= 2, within 1 ulp: the FP32 reciprocal of its leading
+// bits (2^-20) and one step of Newton's iteration, third order.
+__device__ __forceinline__ double reciprocal_1_2(double s) {
+  const float f = __uint_as_float(__funnelshift_l(__double2loint(s), __double2hiint(s), 3) + 0x40000000u);
+  float g;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(g) : "f"(f));
+  const double r = __hiloint2double((int)((__float_as_uint(g) >> 3) + 0x38000000u), 0);
+  const double e = fma(-s, r, 1.0);
+  return fma(r, fma(e, e, e), r);
 }
 
 __global__ void __launch_bounds__(kMixWarps * 32, 1) gamma_fit_kernel(const double* __restrict__ hist, int64_t n, int bins,
                                                                      float t0, float bw,
                                                                      const float* __restrict__ tshift,
                                                                      float* __restrict__ out, int iters) {
-  extern __shared__ double mix_smem[];
+  extern __shared__ double2 mix_smem[];
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // the filled bins: weight, log time, bin (a pair's bins from 65536 on are not gathered)
-  double* const eh = mix_smem + (size_t)warp * kMixEntries * 2;
-  double* const el = eh + kMixEntries;
-  uint16_t* const eb = reinterpret_cast<uint16_t*>(mix_smem + (size_t)kMixWarps * kMixEntries * 2) + warp * kMixEntries;
+  double2* const entry = mix_smem + (size_t)warp * kMixEntries;  // the filled bins: weight, log time
   // the block's pairs are blockIdx.x + i gridDim.x; its warps take them from a
   // counter, at most a warp's share of what is left at a time
   __shared__ unsigned taken;
   if (threadIdx.x == 0) taken = 0;
   __syncthreads();
+  const ppsf::WarpTables T = ppsf::warp_tables();
   const int64_t mine = (n - blockIdx.x + gridDim.x - 1) / gridDim.x;
   auto take = [&]() {
     unsigned i = 0;
@@ -1031,20 +1054,30 @@ __global__ void __launch_bounds__(kMixWarps * 32, 1) gamma_fit_kernel(const doub
   int64_t next = take();
   while (next < mine) {
     const int share = (int)min((int64_t)kMixPairs, (mine - next + kMixWarps - 1) / kMixWarps);
+    bool held = true;  // `next` is not fitted yet
     // this lane's pair (lane / 2) and component (lane % 2; 0 is the one with the smaller start value)
     int64_t pair = -1;
     int first = 0, count = 0, rest = bins;  // entries in shared memory; bins from `rest` on are read again
-    double s0 = 0, a = 1, w = 0.5, th = 1;
+    double s0 = 0, st = 0, a = 1, w = 0.5, th = 1;  // sums of the weights and of weight x time
     int used = 0, m = 0;
-    for (; m < share && next < mine; ++m, next = take()) {
+    for (; m < share; ++m) {
+      if (!held) next = take();
+      held = true;
+      if (next >= mine) break;
       const int64_t row = blockIdx.x + next * gridDim.x;
       const double* h = hist + row * bins;
       const double ts = tshift[row];
       double p0 = 0, p1 = 0, p2 = 0;
       int k = 0, b0 = 0, stop = bins;
+      auto ahead = [&](unsigned b) { return b < (unsigned)bins ? h[b] : 0.0; };
+      double h1 = ahead(lane), h2 = ahead(32 + lane), h3 = ahead(64 + lane), h4 = ahead(96 + lane);
       for (; b0 < bins; b0 += 32) {
         const int b = b0 + lane;
-        const double hb = b < bins ? h[b] : 0.0, t = t0 + (b + 0.5) * bw - ts;
+        const double hb = h1, t = t0 + (b + 0.5) * bw - ts;
+        h1 = h2;
+        h2 = h3;
+        h3 = h4;
+        h4 = ahead(b + 128u);
         const bool in = t > 0 && hb > 0;
         const unsigned ball = __ballot_sync(kAll, in);
         if (!ball) continue;
@@ -1053,16 +1086,13 @@ __global__ void __launch_bounds__(kMixWarps * 32, 1) gamma_fit_kernel(const doub
           p1 += hb * t;
           p2 += hb * t * t;
         }
-        if (stop < bins || used + k + __popc(ball) > kMixEntries || b0 > 65535 - 32) {
+        if (stop < bins || used + k + __popc(ball) > kMixEntries) {
           stop = min(stop, b0);
           if (m > 0) break;  // the pair opens the next round
           continue;
         }
         if (in) {
-          const int at = used + k + __popc(ball & ((1u << lane) - 1u));
-          eh[at] = hb;
-          el[at] = log(t);
-          eb[at] = (uint16_t)b;
+          entry[used + k + __popc(ball & ((1u << lane) - 1u))] = make_double2(hb, log(t));
         }
         k += __popc(ball);
       }
@@ -1076,71 +1106,89 @@ __global__ void __launch_bounds__(kMixWarps * 32, 1) gamma_fit_kernel(const doub
         count = k;
         rest = stop;
         s0 = p0;
+        st = p1;
         const double mean = p1 / p0, v = fmax(p2 / p0 - mean * mean, 1e-6 * mean * mean + 1e-12);
         const double a0 = fmax(mean * mean / v, 0.05);
         a = (lane & 1) ? 2.0 * a0 : fmax(0.5 * a0, 0.02);
         th = v / mean;
       }
       used += k;
+      held = false;
     }
     __syncwarp();
     const bool live = pair >= 0 && s0 > 0;
     if (!live) a = th = 1.0;  // harmless values for the lanes without a fit
-    double ll = 0;
+    Psi P;
+    P.eval(a);
+    double ll = 0, lth = log(th);
 #pragma unroll 1
     for (int it = 0; it < iters; ++it) {
-      const double lth = log(th), lw = (lane & 1) ? log1p(-w) : log(w);
-      const double c = lw - a * lth - lgamma(a);
+      const double c = log((lane & 1) ? 1.0 - w : w) - a * lth - lgamma(a);
       const double cd = c - __shfl_xor_sync(kAll, c, 1), ad = a - __shfl_xor_sync(kAll, a, 1);
-      double S0 = 0, S1 = 0, SL = 0;  // this lane's component
+      double S0 = 0, SL = 0;  // this lane's component
 #pragma unroll 1
       for (int p = 0; p < m; ++p) {
         // log ratio of component 1's density to component 2's: da lt + dc (even lanes hold component 1)
         const double dc = __shfl_sync(kAll, cd, 2 * p), da = __shfl_sync(kAll, ad, 2 * p);
         const int f0 = __shfl_sync(kAll, first, 2 * p), k = __shfl_sync(kAll, count, 2 * p);
         const int stop = __shfl_sync(kAll, rest, 2 * p);
-        const int64_t row = __shfl_sync(kAll, pair, 2 * p);
-        const double ts = tshift[row];
-        double q0 = 0, q1 = 0, q2 = 0, r0 = 0, r1 = 0, r2 = 0;
-        auto add = [&](double hb, double t, double lt) {
-          const double d = fma(da, lt, dc);
-          const double e = exp(-fabs(d)), v = 1.0 / (1.0 + e);
-          const double f = d > 0 ? v : e * v;  // component 1's share
-          // 1 - f, which is 0 once component 2 falls below the rounding of 1:
-          // its parameters then stay as they are
-          const double x = hb * f, y = hb * (1.0 - f);
-          q0 += x;
-          q1 = fma(x, t, q1);
-          q2 = fma(x, lt, q2);
-          r0 += y;
-          r1 = fma(y, t, r1);
-          r2 = fma(y, lt, r2);
+        double q0 = 0, q2 = 0, r0 = 0, r2 = 0;
+        auto add = [&](auto... h_lt) {  // all lanes
+          constexpr int Q = sizeof...(h_lt);
+          const double2 in[Q] = {h_lt...};
+          double d[Q], e[Q];
+          bool far = false;  // beyond the table's range
+#pragma unroll
+          for (int q = 0; q < Q; ++q) {
+            d[q] = fma(da, in[q].y, dc);
+            e[q] = ppsf::exp_tab(-fabs(d[q]), T);
+            far = far || (__double2hiint(d[q]) & 0x7fffffff) >= 0x40862000;
+          }
+          if (__any_sync(kAll, far)) {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) e[q] = exp(-fabs(d[q]));
+          }
+#pragma unroll
+          for (int q = 0; q < Q; ++q) {
+            const double v = reciprocal_1_2(1.0 + e[q]);
+            const double f = d[q] > 0 ? v : e[q] * v;  // component 1's share
+            // 1 - f, which is 0 once component 2 falls below the rounding of 1:
+            // its parameters then stay as they are
+            const double x = in[q].x * f, y = in[q].x * (1.0 - f);
+            q0 += x;
+            q2 = fma(x, in[q].y, q2);
+            r0 += y;
+            r2 = fma(y, in[q].y, r2);
+          }
         };
-#pragma unroll 2
-        for (int i = f0 + lane; i < f0 + k; i += 32) add(eh[i], t0 + (eb[i] + 0.5) * bw - ts, el[i]);
-        if (stop < bins) {  // what did not fit
-          const double* h = hist + row * bins;
+        const double2 none = make_double2(0.0, 0.0);
+        int i = lane;
 #pragma unroll 1
-          for (int b = stop + lane; b < bins; b += 32) {
-            const double hb = h[b], t = t0 + (b + 0.5) * bw - ts;
-            if (t > 0 && hb > 0) add(hb, t, log(t));
+        for (; i - lane + 32 < k; i += 64) add(entry[f0 + i], i + 32 < k ? entry[f0 + i + 32] : none);
+        if (i - lane < k) add(i < k ? entry[f0 + i] : none);
+        if (stop < bins) {  // what did not fit
+          const int64_t row = __shfl_sync(kAll, pair, 2 * p);
+          const double* h = hist + row * bins;
+          const double ts = tshift[row];
+#pragma unroll 1
+          for (int b0 = stop; b0 < bins; b0 += 32) {
+            const int b = b0 + lane;
+            const double hb = b < bins ? h[b] : 0.0, t = t0 + (b + 0.5) * bw - ts;
+            add(t > 0 && hb > 0 ? make_double2(hb, log(t)) : none);
           }
         }
         // even lanes sum component 1, odd lanes component 2
         const bool odd = lane & 1;
-        double u0 = odd ? r0 : q0, u1 = odd ? r1 : q1, u2 = odd ? r2 : q2;
+        double u0 = odd ? r0 : q0, u2 = odd ? r2 : q2;
         u0 += __shfl_xor_sync(kAll, odd ? q0 : r0, 1);
-        u1 += __shfl_xor_sync(kAll, odd ? q1 : r1, 1);
         u2 += __shfl_xor_sync(kAll, odd ? q2 : r2, 1);
 #pragma unroll
         for (int o = 2; o < 32; o <<= 1) {
           u0 += __shfl_xor_sync(kAll, u0, o);
-          u1 += __shfl_xor_sync(kAll, u1, o);
           u2 += __shfl_xor_sync(kAll, u2, o);
         }
         if ((lane >> 1) == p) {
           S0 = u0;
-          S1 = u1;
           SL = u2;
         }
       }
@@ -1149,40 +1197,49 @@ __global__ void __launch_bounds__(kMixWarps * 32, 1) gamma_fit_kernel(const doub
         for (int p = 0; p < m; ++p) {
           const double dc = __shfl_sync(kAll, cd, 2 * p), da = __shfl_sync(kAll, ad, 2 * p);
           const double c2 = __shfl_sync(kAll, c, 2 * p + 1), a2 = __shfl_sync(kAll, a, 2 * p + 1);
-          const double rth = 1.0 / __shfl_sync(kAll, th, 2 * p);
-          const int64_t row = __shfl_sync(kAll, pair, 2 * p);
-          const double* h = hist + row * bins;
-          const double ts = tshift[row];
+          const int f0 = __shfl_sync(kAll, first, 2 * p), k = __shfl_sync(kAll, count, 2 * p);
+          const int stop = __shfl_sync(kAll, rest, 2 * p);
           double L = 0;
+          auto add = [&](double hb, double lt) {
+            const double d = fma(da, lt, dc);
+            L += hb * (fma(a2 - 1.0, lt, c2) + fmax(d, 0.0) + log1p(exp(-fabs(d))));
+          };
 #pragma unroll 1
-          for (int b = lane; b < bins; b += 32) {
-            const double hb = h[b], t = t0 + (b + 0.5) * bw - ts;
-            if (!(t > 0) || !(hb > 0)) continue;
-            const double lt = log(t), d = fma(da, lt, dc);
-            L += hb * (fma(a2 - 1.0, lt, c2) - t * rth + fmax(d, 0.0) + log1p(exp(-fabs(d))));
+          for (int i = f0 + lane; i < f0 + k; i += 32) add(entry[i].x, entry[i].y);
+          if (stop < bins) {
+            const int64_t row = __shfl_sync(kAll, pair, 2 * p);
+            const double* h = hist + row * bins;
+            const double ts = tshift[row];
+#pragma unroll 1
+            for (int b = stop + lane; b < bins; b += 32) {
+              const double hb = h[b], t = t0 + (b + 0.5) * bw - ts;
+              if (t > 0 && hb > 0) add(hb, log(t));
+            }
           }
           L = warp_sum(L);
-          if ((lane >> 1) == p) ll = L / s0;
+          if ((lane >> 1) == p) ll = (L - st / th) / s0;
         }
       }
       const double o0 = __shfl_xor_sync(kAll, S0, 1);
-      const double S1t = S1 + __shfl_xor_sync(kAll, S1, 1);
       const double wa = (lane & 1) ? o0 : S0, wb = (lane & 1) ? S0 : o0;
       if (live) w = fmin(fmax(wa / (wa + wb), 1e-4), 1 - 1e-4);
       const bool solve = live && S0 > 0;
 #pragma unroll 1
       for (int j = 0; j < 3; ++j) {
         const double v = a * S0, vt = v + __shfl_xor_sync(kAll, v, 1);
-        if (live) th = S1t / vt;
-        const double y = solve ? SL / S0 - log(th) : 0.0;
-        const double an = inv_digamma(y, a, solve);
+        if (live) th = st / vt;
+        lth = log(th);
+        const double y = solve ? SL / S0 - lth : 0.0;
+        const double an = inv_digamma(y, P, solve);
         if (solve) a = an;
       }
     }
     const double oa = __shfl_xor_sync(kAll, a, 1);
     if (pair >= 0 && !(lane & 1)) {
       float* o = out + pair * 5;
-      const bool swap = a > oa;  // order the components
+      // order the components, by the shapes as they are returned: where the two
+      // have met but for rounding (1 % of pairs with a few filled bins), the order stays
+      const bool swap = (float)a > (float)oa;
       const float nan = __int_as_float(0x7fc00000);
       o[0] = live ? (float)(swap ? 1 - w : w) : nan;
       o[1] = live ? (float)(swap ? oa : a) : nan;
@@ -1191,6 +1248,7 @@ __global__ void __launch_bounds__(kMixWarps * 32, 1) gamma_fit_kernel(const doub
       o[4] = live ? (float)ll : nan;
     }
     __syncwarp();
+    if (!held) next = take();
   }
 }
 
