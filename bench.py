@@ -974,7 +974,7 @@ def run_ours(args):
     f_mufu, f_fp32 = a_mufu / peaks["mufu_ops"], a_fp32 / peaks["fp32_ops"]
     hits_local = int(cnt[:, 0].sum())
     # algorithmic HBM bytes over the K steps: pairs in, hits out, histograms and statistics zeroed and written,
-    # chunk offsets written and read
+    # queue offsets written and read
     alg_bytes = K * (n_pairs * 80 + 2 * n_pairs * (bins + 8) * 8 + 2 * (n_pairs + 1) * 8) + hits_local * 64
 
     # plain: one launch per pair on the same batch, kernels only (no host sync

@@ -134,7 +134,7 @@ typedef struct {
   uint32_t flags;     /* PP_OPT_* */
   int32_t block_size; /* launch tuning; 0 = autotuned/default */
   int32_t blocks_per_sm;
-  int32_t chunk_photons;
+  int32_t chunk_photons; /* photons a warp takes from the work queue at once, at most */
   int32_t reserved;
 } pp_run_opts;
 
@@ -203,7 +203,7 @@ PP_API pp_status pp_get_knots(const pp_ctx* ctx, float* out, int32_t cap, int32_
 
 /* ---- hot path ------------------------------------------------------------ */
 /* Batched persistent kernel over all pairs (device work queue of photon
- * chunks), host buffers, synchronous.  Replaces propagate_distance
+ * ranges), host buffers, synchronous.  Replaces propagate_distance
  * (src/photon_prop_cuda.jl:588-644) for any number of source-target pairs.
  * hits: hit_capacity records (may be NULL with capacity 0); stats:
  * n_pairs x PP_STATS doubles; hist: n_pairs x hist_bins doubles (NULL if
@@ -236,7 +236,7 @@ PP_API pp_status pp_propagate_device(pp_ctx* ctx, const pp_pair* d_pairs, int64_
  * CUDA.jl allocator or PyTorch's caching allocator may hold the free memory,
  * so a library cudaMalloc can fail, and cudaMalloc/cudaFree can synchronise
  * the device in the middle of the caller's stream work.  The work-queue
- * scratch (chunk offsets and queue cursor) lives in one static device array
+ * scratch (pair offsets and queue cursor) lives in one static device array
  * of (PP_NOALLOC_MAX_PAIRS + 33) x 8 bytes (about 512 KiB) that every GPU
  * which loads the library holds until the process exits.  The call allocates
  * nothing, launches directly (no graph) and otherwise behaves like

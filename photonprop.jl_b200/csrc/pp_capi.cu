@@ -1252,7 +1252,7 @@ cudaError_t ctx_llh_scratch(pp_ctx* c, size_t bytes, void** out) {
 // Allocation-free batched propagation (pp_propagate_device_noalloc).
 //
 // The work-queue scratch is this file-scope device array: word 0 is the queue
-// cursor, words 32.. the chunk offsets (n_pairs + 1 of them).  In host code
+// cursor, words 32.. the pairs' offsets in the queue (n_pairs + 1 of them).  In host code
 // the name g_noalloc_scratch is only a host-side stand-in for the symbol, not
 // a device address: a kernel given it would fault or, where the GPU can reach
 // host memory, silently use the wrong memory.  The device address is looked
@@ -1313,7 +1313,7 @@ extern "C" pp_status pp_propagate_device_noalloc(pp_ctx* c, const pp_pair* d_pai
   a.counters = reinterpret_cast<unsigned long long*>(d_counters);
   a.stats = d_stats;
   a.hist = opts->hist_bins > 0 ? d_hist : nullptr;
-  // the scan kernel rewrites every offset and zeroes the cursor and counters
+  // the set-up kernel rewrites every offset and zeroes the cursor and counters
   if ((e = enqueue_batched(c, a, grid, block, static_cast<cudaStream_t>(stream))))
     return c->cuda_fail(e, "pp_propagate_device_noalloc");
   return PP_OK;

@@ -48,11 +48,11 @@ def op_counts(steps, photons_iso, photons_cone, algorithmic=False):
 # DRAM traffic of one launch of the 4096-pair benchmark batch (5.75e9
 # photons), full size, `--metrics dram__bytes_read.sum,dram__bytes_write.sum
 # --cache-control none` (one pass): the two timed launches after an L2 flush
-# read 2.3 and 3.0 MB and wrote 23.1 and 32.8 MB.  The rest of a step's
+# read 2.1 and 2.6 MB and wrote 22.3 and 30.9 MB.  The rest of a step's
 # algorithmic bytes (zeroed and accumulated FP64 histograms, hit records)
 # stays in the 126 MB L2 during the launch and reaches DRAM afterwards.
-NCU_DRAM_BYTES_PER_LAUNCH = 0.5 * ((2.27 + 23.11) + (3.04 + 32.76)) * 1e6
+NCU_DRAM_BYTES_PER_LAUNCH = 0.5 * ((2.08 + 22.35) + (2.57 + 30.91)) * 1e6
 # Issue and pipes on one launch of 512 mixed pairs (<= 1e6 photons each).
-NCU_ISSUE_ACTIVE = 0.779
-NCU_PIPES = {"alu": 0.518, "fma": 0.395, "xu": 0.375}  # pipe utilisation, same capture
-NCU_LANES_ACTIVE = 29.97  # threads per executed warp instruction, same capture
+NCU_ISSUE_ACTIVE = 0.777
+NCU_PIPES = {"alu": 0.478, "fma": 0.421, "xu": 0.406}  # pipe utilisation, same capture
+NCU_LANES_ACTIVE = 30.59  # threads per executed warp instruction, same capture
