@@ -337,15 +337,16 @@ __device__ __forceinline__ void rotate_to_axis(float ox, float oy, float oz, flo
 struct RunParams {
   const pp_pair* __restrict__ pairs;
   int64_t n_pairs;
-  const unsigned long long* __restrict__ granule_offsets;  // [n_pairs + 1] first 32-photon granule of each pair
-  unsigned long long* __restrict__ queue;                  // [0]: next granule
+  // no __restrict__ on what the set-up and fill kernels write while the batched kernel starts
+  const unsigned long long* granule_offsets;  // [n_pairs + 1] first 32-photon granule of each pair
+  unsigned long long* queue;                  // [0]: next granule
   uint32_t max_run;  // granules a warp takes at once, at most
   uint32_t pair_base;  // added to the pair index written into hits
   pp_hit* __restrict__ hits;
   unsigned long long hit_cap;
-  unsigned long long* __restrict__ counters;  // [0] hits, [1] steps, [2] status bits
-  double* __restrict__ stats;                 // [n_pairs x PP_STATS]
-  double* __restrict__ hist;                  // [n_pairs x hist_bins]
+  unsigned long long* counters;  // [0] hits, [1] steps, [2] status bits
+  double* stats;                 // [n_pairs x PP_STATS]
+  double* hist;                  // [n_pairs x hist_bins]
   const DevTables* __restrict__ tables;
   int32_t max_steps;
   uint32_t ctr_limit;  // (max_steps + 1) << 8: a photon whose next counter word reaches it has ended

@@ -151,8 +151,7 @@ __global__ void __launch_bounds__(kThreads, 6) llh_kernel(int mode, int64_t S, i
                                                        const double* __restrict__ photons,
                                                        const int64_t* __restrict__ offsets,
                                                        const double* __restrict__ times,
-                                                       const int64_t* __restrict__ chunk_start,
-                                                       double* __restrict__ llh) {
+                                                       const int64_t* chunk_start, double* llh) {
   __shared__ Term terms[kTile];
   __shared__ double part[kWarps][kBlockHits];
   __shared__ double red[kWarps];

@@ -44,7 +44,10 @@ void count_launches(uint64_t n);
 
 // A launch that may start while the kernel before it on the stream runs (its
 // programmatic dependent): it waits itself, by griddepcontrol.wait, before it
-// reads what that kernel writes.
+// reads what that kernel writes.  Its pointers to that data are not
+// __restrict__: the qualifier promises that nobody else writes them while the
+// kernel runs, on which a load may be moved above the wait or go through the
+// read-only path.
 template <typename... P, typename... A>
 cudaError_t launch_dependent(void (*fn)(P...), dim3 grid, int block, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};

@@ -580,8 +580,7 @@ constexpr int kGradPitch = 528;  // bytes of a staged gradient row: 16-byte lane
 __global__ void __launch_bounds__(TRAIN_THREADS, 1) train_kernel(DevParams P, const float* __restrict__ xn,
                                                                 const float* __restrict__ yt,
                                                                 const float* __restrict__ mask, int64_t n,
-                                                                const double* __restrict__ part,
-                                                                float* __restrict__ grad) {
+                                                                const double* part, float* grad) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // W2 H1 W3 H2 DZ3 DZ2, 32 KB each; reused as they fall free:
   unsigned char* const base = smem_raw;
@@ -906,7 +905,7 @@ __device__ __forceinline__ void write_copies(const Copies& C, int i, float v) {
 }
 
 // Adam on the FP32 master parameters, and their BF16 copies.
-__global__ void __launch_bounds__(256) adam_kernel(float* __restrict__ p, const float* __restrict__ g,
+__global__ void __launch_bounds__(256) adam_kernel(float* __restrict__ p, const float* g,
                                                    float* __restrict__ m, float* __restrict__ v, const Copies C,
                                                    float lr, float b1, float b2, float eps, float c1, float c2) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
