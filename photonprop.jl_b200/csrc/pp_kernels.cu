@@ -185,6 +185,7 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
   // lookup per 4096 photons), short ones at the end, so that the warps finish
   // together, and a small batch spreads over all of them.
   auto fetch = [&]() {
+    __syncwarp();  // every lane has read the run and added its hits' sums before lane 0 writes them
     int p = -1;
     if (lane == 0) {
       unsigned long long at = wa->run_at, end = wa->run_end;
