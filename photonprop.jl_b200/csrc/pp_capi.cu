@@ -123,7 +123,7 @@ struct pp_ctx {
   // buffers of the host-buffer entry points; `out` holds pp_propagate's
   // counters, statistics and histograms one after the other
   DevBuf pairs, hits, counters, stats, hist, out;
-  unsigned char* stage = nullptr;  // pinned, kStageBytes: what a small call copies in and out
+  unsigned char* stage = nullptr;  // pinned, kStageBytes: what a small call copies in and out (NULL: nothing is staged)
   // work-queue scratch of the batched kernel
   DevBuf offsets, queue;
   // launch shape per mode (0 = resolve at launch)
@@ -463,15 +463,17 @@ pp_status pp_create(pp_ctx** out, int device, const pp_medium_desc* medium, cons
   }
   if ((e = cudaMalloc(&c->d_tables, c->h_tables.size())) ||
       (e = cudaMemcpy(c->d_tables, c->h_tables.data(), c->h_tables.size(), cudaMemcpyHostToDevice)) ||
-      (e = cudaHostAlloc(&c->stage, kStageBytes, cudaHostAllocDefault)) ||
       (e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking))) {
     g_create_error = std::string("pp_create: ") + cudaGetErrorString(e);
     cudaGetLastError();
     if (c->d_tables) cudaFree(c->d_tables);
-    if (c->stage) cudaFreeHost(c->stage);
     cudaFree(c->d_casc);
     delete c;
     return e == cudaErrorMemoryAllocation ? PP_ERR_OOM : PP_ERR_CUDA;
+  }
+  if (cudaHostAlloc(&c->stage, kStageBytes, cudaHostAllocDefault)) {  // no pinned memory left: every call copies directly
+    cudaGetLastError();
+    c->stage = nullptr;
   }
   *out = c;
   return PP_OK;
@@ -572,9 +574,9 @@ pp_status pp_propagate(pp_ctx* c, const pp_pair* pairs, int64_t n_pairs, const p
     return alloc_fail(c, e, "pp_propagate buffers");
   if (grew) c->drop_graphs();
   cudaStream_t s = c->stream;
-  const bool staged = in_bytes <= kStageIn && out_bytes <= kStageOut;
-  unsigned char* const stage_out = c->stage + kStageIn;
-  unsigned char* const stage_hits = stage_out + kStageOut;
+  const bool staged = c->stage && in_bytes <= kStageIn && out_bytes <= kStageOut;
+  unsigned char* const stage_out = staged ? c->stage + kStageIn : nullptr;
+  unsigned char* const stage_hits = staged ? stage_out + kStageOut : nullptr;
   unsigned char* const d_out = static_cast<unsigned char*>(c->out.p);
   const void* src = pairs;
   if (staged && n_pairs > 0) {
