@@ -221,7 +221,9 @@ PP_API pp_status pp_propagate_plain(pp_ctx* ctx, const pp_pair* pairs, int64_t n
 
 /* Device-buffer, asynchronous form of pp_propagate on `stream` (a
  * cudaStream_t; NULL = legacy default stream).  counters: 4 uint64 on the
- * device, [0] = total hits, [1] = photon steps taken, [2] = status bits
+ * device, [0] = total hits, [1] = photon steps of the model (in physical mode
+ * a step that would only find its photon out of reach counts, though it is
+ * not made: pp_made_steps_device), [2] = status bits
  * (1 = hit overflow), [3] reserved; they are reset by the call.  The work
  * queue lives in context-owned device scratch memory.  Repeated calls with
  * the same shapes and buffers replay a captured CUDA graph. */
@@ -556,6 +558,13 @@ PP_API pp_status pp_measure_peaks(int device, double* fp32_ops_per_s, double* mu
  * occupancy.  No reference counterpart: the ceiling the batched kernel's
  * step rate is reported against. */
 PP_API pp_status pp_measure_step_rate(int device, double* steps_per_s);
+
+/* Photon steps that a propagation of these pairs (device buffer) makes, which
+ * is what a step rate of the kernels is: the photon steps of counters[1]
+ * without those that the reach test of the physical mode spares.  Simulates
+ * the pairs again, recording nothing; synchronous.  No reference counterpart. */
+PP_API pp_status pp_made_steps_device(pp_ctx* ctx, const pp_pair* d_pairs, int64_t n_pairs,
+                                      const pp_run_opts* opts, uint64_t* made);
 
 #ifdef __cplusplus
 }

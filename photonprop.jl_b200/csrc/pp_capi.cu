@@ -778,6 +778,34 @@ pp_status pp_cuda_propagate_photons(pp_ctx* c, float* pos, float* dir, float* wl
   return PP_OK;
 }
 
+pp_status pp_made_steps_device(pp_ctx* c, const pp_pair* d_pairs, int64_t n_pairs, const pp_run_opts* opts,
+                               uint64_t* made) {
+  if (!c) return PP_ERR_ARG;
+  std::lock_guard<std::mutex> lk(c->mu);
+  pp_status st = validate_opts(c, opts);
+  if (st) return st;
+  if (n_pairs < 0 || n_pairs > (int64_t)INT32_MAX || (n_pairs > 0 && !d_pairs) || !made || !aligned(d_pairs, 16))
+    return c->fail(PP_ERR_ARG, "pp_made_steps_device: bad arguments");
+  *made = 0;
+  if (n_pairs == 0) return PP_OK;
+  DeviceGuard guard(c->device);
+  unsigned long long* d_made = nullptr;
+  cudaError_t e;
+  if ((e = cudaMalloc(&d_made, sizeof *d_made))) return alloc_fail(c, e, "pp_made_steps_device");
+  pp::LaunchArgs a = base_args(c, opts);
+  a.pairs = d_pairs;
+  a.n_pairs = n_pairs;
+  unsigned long long v = 0;
+  if (!(e = cudaMemsetAsync(d_made, 0, sizeof *d_made, c->stream)) &&
+      !(e = pp::launch_made_steps(a, d_made, c->sm_count, c->stream)) &&
+      !(e = cudaMemcpyAsync(&v, d_made, sizeof v, cudaMemcpyDeviceToHost, c->stream)))
+    e = cudaStreamSynchronize(c->stream);
+  cudaFree(d_made);
+  if (e) return c->cuda_fail(e, "pp_made_steps_device");
+  *made = v;
+  return PP_OK;
+}
+
 pp_status pp_device_eval(pp_ctx* c, int32_t op, const double* in, double* out, int64_t n) {
   if (!c) return PP_ERR_ARG;
   std::lock_guard<std::mutex> lk(c->mu);

@@ -84,6 +84,8 @@ cudaError_t launch_plain(const LaunchArgs& a, const pp_pair* d_pair, int pair_in
 cudaError_t launch_stacks(const LaunchArgs& a, const pp_pair* d_pair, float* pos, float* dir, float* wl,
                           float* dist, int32_t* sp, int64_t* nsim, int stack_len, int grid, int block,
                           long long per_thread, cudaStream_t s);
+// Adds the step events that a propagation makes to *out (n_pairs >= 1).
+cudaError_t launch_made_steps(const LaunchArgs& a, unsigned long long* out, int sm_count, cudaStream_t s);
 cudaError_t launch_normalize(const pp_pair* pairs, int64_t n, double* hist, int bins, int sm_count, cudaStream_t s);
 cudaError_t launch_eval(int op, const double* in, double* out, int64_t n, const void* tables, cudaStream_t s);
 int batched_max_blocks_per_sm(int mode, int block, bool cascade);

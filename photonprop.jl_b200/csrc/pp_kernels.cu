@@ -392,6 +392,37 @@ __global__ void __launch_bounds__(512) plain_kernel(const RunParams R, const pp_
 }
 
 // ---------------------------------------------------------------------------
+// Step events that a propagation of these pairs makes: counters[1] counts the
+// step that would only find a photon out of reach, which no kernel makes.
+// A diagnostic of the rates' denominators (one thread per photon, nothing
+// recorded), so that the batched kernel need not count both.
+template <int MODE, int EM>
+__global__ void __launch_bounds__(256) made_steps_kernel(const RunParams R, unsigned long long* __restrict__ out) {
+  __shared__ __align__(16) DevTables T;
+  stage_tables(T, R.tables);
+  __syncthreads();
+  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+  unsigned long long made = 0;
+  for (int64_t p = blockIdx.y; p < R.n_pairs; p += gridDim.y) {
+    const PairCtx c{R.pairs[p].radius, (int)p};
+    const long long photons = R.pairs[p].n_photons;
+    const unsigned long long n = photons > 0 ? (unsigned long long)photons : 0ull;
+    for (unsigned long long id = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; id < n; id += stride) {
+      Photon s;
+      set_photon(s, id);
+      bool hit, more, alive = emit_event<MODE, EM>(T, R, load_pair(R.pairs + p), s);
+      for (; alive; ++made) {
+        alive = step_event<MODE>(R, c, s, hit, more);
+        if (MODE == kCompat) alive = more;
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) made += __shfl_xor_sync(kFull, made, o);
+  if ((threadIdx.x & 31u) == 0) atomicAdd(out, made);
+}
+
+// ---------------------------------------------------------------------------
 // cuda_propagate_photons! layout (src/photon_prop_cuda.jl:262-386).  Photon
 // ids: thread g simulates ids g + i * (blocks * threads), i < per_thread.
 template <int MODE>
@@ -853,6 +884,21 @@ cudaError_t launch_plain(const LaunchArgs& a, const pp_pair* d_pair, int pair_in
     ppd::plain_kernel<ppd::kPhysical, ppd::kEmCascade><<<grid, block, 0, s>>>(R, d_pair, pair_index);
   else
     ppd::plain_kernel<ppd::kPhysical, ppd::kEmBasic><<<grid, block, 0, s>>>(R, d_pair, pair_index);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_made_steps(const LaunchArgs& a, unsigned long long* out, int sm_count, cudaStream_t s) {
+  const ppd::RunParams R = to_params(a);
+  // 32 blocks per SM where the pairs are few, one per pair where they are many
+  const int64_t rows = std::min<int64_t>(a.n_pairs, 32768);
+  const dim3 grid((unsigned)std::max<int64_t>(1, 32 * (int64_t)sm_count / rows), (unsigned)rows);
+  if (a.opts.mode == PP_MODE_COMPAT)
+    ppd::made_steps_kernel<ppd::kCompat, ppd::kEmBasic><<<grid, 256, 0, s>>>(R, out);
+  else if (a.opts.flags & PP_OPT_CASCADE)
+    ppd::made_steps_kernel<ppd::kPhysical, ppd::kEmCascade><<<grid, 256, 0, s>>>(R, out);
+  else
+    ppd::made_steps_kernel<ppd::kPhysical, ppd::kEmBasic><<<grid, 256, 0, s>>>(R, out);
   count_launches(1);
   return cudaGetLastError();
 }

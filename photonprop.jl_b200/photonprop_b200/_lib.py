@@ -166,6 +166,7 @@ _SIGS = [
     ("pp_gamma_mixture_fit", ctypes.c_int, [_VP, _I64, _I32, ctypes.c_float, ctypes.c_float, _VP, _VP, _I32, _VP]),
     ("pp_autotune", ctypes.c_int, [_VP, _VP, _I64, ctypes.POINTER(RunOpts), ctypes.c_char_p,
                                    ctypes.POINTER(RunOpts), ctypes.POINTER(_D)]),
+    ("pp_made_steps_device", ctypes.c_int, [_VP, _VP, _I64, ctypes.POINTER(RunOpts), ctypes.POINTER(ctypes.c_uint64)]),
     ("pp_device_eval", ctypes.c_int, [_VP, _I32, _VP, _VP, _I64]),
     ("pp_measure_peaks", ctypes.c_int, [ctypes.c_int, ctypes.POINTER(_D), ctypes.POINTER(_D),
                                         ctypes.POINTER(_D)]),

@@ -238,6 +238,15 @@ class Propagator:
         return {"block_size": best.block_size, "blocks_per_sm": best.blocks_per_sm,
                 "chunk_photons": best.chunk_photons, "photons_per_s": rate.value}
 
+    def made_steps(self, d_pairs, n_pairs, opts: RunOptions) -> int:
+        """Photon steps that a propagation of these pairs (a device buffer) makes: its step counter without the
+        steps that the physical mode's reach test spares (pp_made_steps_device)."""
+        o = opts.to_c()
+        n = ctypes.c_uint64()
+        _lib.check(self._L.pp_made_steps_device(self._h, _lib.ptr(d_pairs), n_pairs, ctypes.byref(o),
+                                                ctypes.byref(n)), self._h)
+        return n.value
+
     def device_eval(self, op: int, inputs) -> np.ndarray:
         out_w = {0: 4, 3: 3, 4: 3, 12: 5}.get(op, 1)
         x = np.ascontiguousarray(inputs, dtype=np.float64)
