@@ -37,7 +37,16 @@ namespace ppd {
 //
 // Compat mode: every photon makes max_steps steps unless it hits, so the 32
 // emitted photons step in lockstep to their end: no ring, no refill, and
-// the lanes of the few that hit idle.
+// the lanes of the few that hit idle.  Where many have hit with many steps
+// still to come (at most kThinLive live lanes, at least kThinSteps steps), the
+// warp goes over to refilling its idle lanes, kRefill or more at a time, until
+// all are idle at once.  One source, 100 steps, 2e8 photons of which 4, 30, 45,
+// 60, 80 % hit at once: 82.6, 83.4, 84.0, 85.1, 85.2 ms in lockstep alone; with
+// the ring that physical mode has 110.5, 87.8, 74.1, 60.6, 42.5 ms; now
+// 80.5, 74.6, 62.3, 48.8, 29.3 ms.  1000 steps, 1e8 photons, 45 and 80 %: 414 and
+// 415 ms, 318 and 125 with the ring, now 291 and 115.  With 10 steps lockstep is
+// the fastest at every share (24.1 against 46.4 ms at 80 %, 4e8 photons), and
+// its kernel without the other loop (THIN) 2 % faster on 2e7 photons.
 //
 // Bound by instruction issue (77 % of the issue slots, ALU half-rate pipe
 // 50 %); what counts is instructions per photon.  512 mixed pairs (1.1e8
@@ -52,6 +61,9 @@ namespace ppd {
 // the first one or two steps of physical mode inside the emission
 // pass (fewer loop iterations, but 180 bytes spilled at 64 registers: 3.26 ms).
 constexpr int kStage = 64;  // >= 2 * 32 - 1 staged emissions per warp (power of two)
+
+constexpr unsigned kThinLive = 20, kRefill = 8;
+constexpr int kThinSteps = 32;
 
 // The ring holds a photon's 16 words as four arrays of 16-byte words, so that
 // neighbouring lanes read and write neighbouring words (one 64-byte record
@@ -95,7 +107,7 @@ struct StagedHit {
 // emitters; the cascade variant's table lookups in the emission block spill
 // at 64, so it gets 80 (768 threads per SM), which runs cone and isotropic
 // pairs as fast as the basic variant does.
-template <int MODE, int WARPS, int EM>
+template <int MODE, int WARPS, int EM, bool THIN = false>
 __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / (WARPS * 32))
     batched_kernel(const RunParams R) {
   __shared__ __align__(16) DevTables T;
@@ -223,21 +235,22 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
     __syncwarp();
     return p >= 0;
   };
-  // emits the pair's next photons, one per lane (lanes past its last photon
-  // emit as well, and drop it); returns whether the lane has one that is in reach
+  // emits the pair's next photons, at most `most`, the lane's the one of its
+  // rank (lanes past the last emit as well, and drop it); returns whether the
+  // lane has one that is in reach
   unsigned steps = 0;  // beyond those that the set-up kernel has counted (physical mode)
-  auto emit = [&](Photon& e, PairCtx& c) {
-    const unsigned left = wa->left, n = min(32u, left);
+  auto emit = [&](Photon& e, PairCtx& c, unsigned rank, unsigned most) {
+    const unsigned left = wa->left, n = min(most, left);
     const uint64_t base = wa->base;
     c.index = wa->pair;
     __syncwarp();
     wa->base = base + n;  // by every lane: the same values
     wa->left = left - n;
-    set_photon(e, base + lane);
+    set_photon(e, base + rank);
     const PairRec P = staged_pair(wa->rec);
     c.r = P.tgt_r.w;
     const bool near = emit_event<MODE, EM>(T, R, P, e);
-    return near && lane < n;
+    return near && rank < n;
   };
 
   if constexpr (MODE == kCompat) {
@@ -245,17 +258,43 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
       if (wa->left == 0u && !fetch()) break;
       Photon s;
       PairCtx c;
-      bool alive = emit(s, c), hit, more;
+      bool alive = emit(s, c, lane, 32u), hit, more, thin = false;
       for (int left = R.max_steps - 1; left > 0; --left) {
         step_event<MODE>(R, c, s, hit, more);
         hit = hit && alive;
         if (take_hits(hit, s, c, left)) {
           alive = alive && !hit;
-          if (!__any_sync(kFull, alive)) break;
+          const unsigned live = __popc(__ballot_sync(kFull, alive));
+          if (THIN) thin = live <= kThinLive && left >= kThinSteps;
+          if (thin || live == 0u) break;
         }
       }
-      step_event<MODE, true>(R, c, s, hit, more);
-      take_hits(hit && alive, s, c, 0);
+      if (!THIN || !thin) {
+        step_event<MODE, true>(R, c, s, hit, more);
+        take_hits(hit && alive, s, c, 0);
+        continue;
+      }
+      bool dry = false;  // the queue is exhausted
+      for (;;) {         // each lane at its photon's own step, until all are done at once
+        const unsigned need = __ballot_sync(kFull, !alive), idle = __popc(need);
+        if (need == kFull) break;
+        if (!dry && idle >= kRefill) {
+          dry = wa->left == 0u && !fetch();
+          if (!dry) {
+            Photon e;
+            PairCtx ec;
+            if (emit(e, ec, __popc(need & lt_mask), idle) && !alive) {
+              s = e;
+              c = ec;
+              alive = true;
+            }
+          }
+        }
+        step_event<MODE>(R, c, s, hit, more);
+        hit = hit && alive;
+        take_hits(hit, s, c, R.max_steps + 1 - (int)(s.ctr3 >> 8));
+        alive = alive && more;
+      }
     }
   } else {
     // warp-uniform state of the ring, and the lane's photon and pair (radius
@@ -304,7 +343,7 @@ __global__ void __launch_bounds__(WARPS * 32, (EM == kEmCascade ? 768 : 1024) / 
         if (wa->left == 0u && !fetch()) break;
         Photon e;
         PairCtx ec;
-        const bool near = emit(e, ec);
+        const bool near = emit(e, ec, lane, 32u);
         const unsigned keep = __ballot_sync(kFull, near);
         if (near) {
           const unsigned slot = (r_head + r_count + __popc(keep & lt_mask)) & (kStage - 1);
@@ -855,10 +894,14 @@ cudaError_t launch_setup(const LaunchArgs& a, int sm_count, cudaStream_t s) {
 
 namespace {
 using BatchedFn = void (*)(ppd::RunParams);
-BatchedFn batched_fn(int mode, int block, bool cascade) {
-  if (mode == PP_MODE_COMPAT)
+BatchedFn batched_fn(int mode, int block, bool cascade, int max_steps = 0) {
+  if (mode == PP_MODE_COMPAT) {
+    if (max_steps > ppd::kThinSteps)  // at least kThinSteps steps can be left
+      return block == 128 ? ppd::batched_kernel<ppd::kCompat, 4, ppd::kEmBasic, true>
+                          : ppd::batched_kernel<ppd::kCompat, 8, ppd::kEmBasic, true>;
     return block == 128 ? ppd::batched_kernel<ppd::kCompat, 4, ppd::kEmBasic>
                         : ppd::batched_kernel<ppd::kCompat, 8, ppd::kEmBasic>;
+  }
   if (cascade)
     return block == 128 ? ppd::batched_kernel<ppd::kPhysical, 4, ppd::kEmCascade>
                         : ppd::batched_kernel<ppd::kPhysical, 8, ppd::kEmCascade>;
@@ -872,7 +915,8 @@ BatchedFn batched_fn(int mode, int block, bool cascade) {
 cudaError_t launch_batched(const LaunchArgs& a, int grid, int block, cudaStream_t s) {
   const ppd::RunParams R = to_params(a);
   if (block != 128) block = 256;
-  return launch_dependent(batched_fn(a.opts.mode, block, (a.opts.flags & PP_OPT_CASCADE) != 0), grid, block, 0, s, R);
+  const auto fn = batched_fn(a.opts.mode, block, (a.opts.flags & PP_OPT_CASCADE) != 0, a.opts.max_steps);
+  return launch_dependent(fn, grid, block, 0, s, R);
 }
 
 cudaError_t launch_plain(const LaunchArgs& a, const pp_pair* d_pair, int pair_index, int grid, int block,
@@ -934,6 +978,7 @@ cudaError_t launch_eval(int op, const double* in, double* out, int64_t n, const 
   return cudaGetLastError();
 }
 
+// (both compat variants have the same registers and shared memory)
 int batched_max_blocks_per_sm(int mode, int block, bool cascade) {
   int nb = 0;
   if (block != 128) block = 256;

@@ -29,7 +29,7 @@ def test_every_dependent_kernel_is_listed():
     for text in _sources().values():
         for m in re.finditer(r"launch_dependent\(\s*([\w:]+)", text):
             names.add(m.group(1).split("::")[-1])
-    assert names - {"batched_fn"} == set(WRITTEN_BEFORE) - {"batched_kernel"}
+    assert names - {"fn"} == set(WRITTEN_BEFORE) - {"batched_kernel"}
 
 
 def test_no_restrict_on_what_the_predecessor_writes():
