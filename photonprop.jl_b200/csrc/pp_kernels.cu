@@ -40,13 +40,15 @@ namespace ppd {
 // the lanes of the few that hit idle.  Where many have hit with many steps
 // still to come (at most kThinLive live lanes, at least kThinSteps steps), the
 // warp goes over to refilling its idle lanes, kRefill or more at a time, until
-// all are idle at once.  One source, 100 steps, 2e8 photons of which 4, 30, 45,
-// 60, 80 % hit at once: 82.6, 83.4, 84.0, 85.1, 85.2 ms in lockstep alone; with
-// the ring that physical mode has 110.5, 87.8, 74.1, 60.6, 42.5 ms; now
-// 80.5, 74.6, 62.3, 48.8, 29.3 ms.  1000 steps, 1e8 photons, 45 and 80 %: 414 and
-// 415 ms, 318 and 125 with the ring, now 291 and 115.  With 10 steps lockstep is
-// the fastest at every share (24.1 against 46.4 ms at 80 %, 4e8 photons), and
-// its kernel without the other loop (THIN) 2 % faster on 2e7 photons.
+// all are idle at once.  One source, 100 steps, 2e8 photons of which 4, 20, 30,
+// 45, 80 % hit at once: 82.6, 83.1, 83.4, 84.0, 85.2 ms in lockstep alone; with
+// the ring that physical mode has 110.5, 97.3, 87.9, 74.2, 42.5 ms; now
+// 80.5, 81.8, 75.2, 62.4, 29.3 ms.  25 steps, 4e8 photons, 20 and 80 %: 43.8 and
+// 48.5 ms, 59.0 and 51.2 with the ring, now 43.7 and 25.5.  kThinLive of 18 or 20
+// costs 2 to 3 % at 20 % hits, where a granule falls below it by chance;
+// kThinSteps of 12 up to 10 % there.  With 10 steps lockstep is twice as
+// fast as the ring at any share (24.1 against 46.4 ms at 80 %), and its kernel
+// without the other loop (THIN) 2 % faster on 2e7 photons.
 //
 // Bound by instruction issue (77 % of the issue slots, ALU half-rate pipe
 // 50 %); what counts is instructions per photon.  512 mixed pairs (1.1e8
@@ -62,8 +64,8 @@ namespace ppd {
 // pass (fewer loop iterations, but 180 bytes spilled at 64 registers: 3.26 ms).
 constexpr int kStage = 64;  // >= 2 * 32 - 1 staged emissions per warp (power of two)
 
-constexpr unsigned kThinLive = 20, kRefill = 8;
-constexpr int kThinSteps = 32;
+constexpr unsigned kThinLive = 16, kRefill = 8;
+constexpr int kThinSteps = 24;
 
 // The ring holds a photon's 16 words as four arrays of 16-byte words, so that
 // neighbouring lanes read and write neighbouring words (one 64-byte record
