@@ -73,11 +73,17 @@ struct DeviceGuard {
 };
 
 // Pinned staging of pp_propagate: a call whose pairs, statistics and
-// histograms fit (1000 pairs, 60 pairs of 1000 bins) makes three copies and one
+// histograms fit (1024 pairs, 65 pairs of 1000 bins) makes three copies and one
 // synchronisation, the first kStageHits hits included; from and to pageable
 // memory they were five copies, each of which waits, and two
-// synchronisations.  One pair of 1e5 photons: 80 us per call before,
-// 48 us now.
+// synchronisations.  One pair of 1e5 photons: 80 us per C call before,
+// 48 us now.  With 1000 photons a pair and 1000 bins, direct against staged:
+// 1 pair 60 and 36 us, 33 pairs 89 and 55, 64 pairs 108 and 70, 100 pairs 128 and
+// 86, 200 pairs 185 and 178, 400 pairs (3.2 MB of results) 285 and 318.  The
+// limit lies at the largest request of the serving workload, well below the
+// point from which the host's second copy costs more than it spares; what lies
+// between takes the direct copies.  Pinning the block costs pp_create 1 to 3 ms
+// of 58.
 constexpr size_t kStageIn = 80 << 10, kStageOut = 512 << 10, kStageHits = 256;
 constexpr size_t kStageBytes = kStageIn + kStageOut + kStageHits * sizeof(pp_hit);
 

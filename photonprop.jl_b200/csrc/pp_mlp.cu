@@ -990,7 +990,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_test_kernel(const __nv_bfloat
 // (one a solve, or none): 2.62 ms.  A pair taken only when there is room for
 // it: 2.53 ms; the histogram loaded four rows ahead: 2.33 ms (issue 55 % of
 // active cycles, FP64 pipe 36 %).  16 warps of 896 bins: 20 of 704 (96
-// registers) took 12 % longer, 24 of 592 17 %.
+// registers) took 12 % longer, 24 of 592 17 %.  Pairs beyond shared memory gain
+// less, and still gain: every bin of 3000 filled, 200, 2000 and 20,000 pairs
+// 6.9, 9.3 and 67.4 ms with one pair per warp, 2.6, 3.1 and 27.5 now; of 10,000,
+// 200 and 2000 pairs 17.9 and 25.8, now 9.2 and 14.7.
 constexpr int kMixWarps = 16, kMixEntries = 896, kMixPairs = 16;
 constexpr size_t kMixSmem = (size_t)kMixWarps * kMixEntries * sizeof(double2);
 
