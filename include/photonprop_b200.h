@@ -542,7 +542,9 @@ PP_API pp_status pp_autotune(pp_ctx* ctx, const pp_pair* pairs, int64_t n_pairs,
  * 7 group index, 8 scattering length, 9 absorption length, 10 PMT
  * acceptance (in: wavelength), 11 cascade-emitter cos theta (in: u, n),
  * 12 a step's Philox2x32-10 block and its three uniforms (in: counter
- * words 0, 1 and the key; out: w0, w1, u0, u1, u2). */
+ * words 0, 1 and the key; out: w0, w1, u0, u1, u2), 13 and 14 the
+ * table-driven FP64 exp and ln, 15 digamma and trigamma (out: 2), 16 the
+ * reciprocal of 1 <= s <= 2. */
 PP_API pp_status pp_device_eval(pp_ctx* ctx, int32_t op, const double* in, double* out, int64_t n);
 
 /* Measures this device's FP32 FMA and MUFU (transcendental) issue peaks with

@@ -815,9 +815,9 @@ pp_status pp_made_steps_device(pp_ctx* c, const pp_pair* d_pairs, int64_t n_pair
 pp_status pp_device_eval(pp_ctx* c, int32_t op, const double* in, double* out, int64_t n) {
   if (!c) return PP_ERR_ARG;
   std::lock_guard<std::mutex> lk(c->mu);
-  static const int in_w[] = {6, 1, 2, 6, 7, 1, 1, 1, 1, 1, 1, 2, 3};
-  static const int out_w[] = {4, 1, 1, 3, 3, 1, 1, 1, 1, 1, 1, 1, 5};
-  if (op < 0 || op > 12 || n < 0 || (n > 0 && (!in || !out))) return c->fail(PP_ERR_ARG, "pp_device_eval: bad arguments");
+  static const int in_w[] = {6, 1, 2, 6, 7, 1, 1, 1, 1, 1, 1, 2, 3, 1, 1, 1, 1};
+  static const int out_w[] = {4, 1, 1, 3, 3, 1, 1, 1, 1, 1, 1, 1, 5, 1, 1, 2, 1};
+  if (op < 0 || op > 16 || n < 0 || (n > 0 && (!in || !out))) return c->fail(PP_ERR_ARG, "pp_device_eval: bad arguments");
   if (n == 0) return PP_OK;
   DeviceGuard guard(c->device);
   double *din = nullptr, *dout = nullptr;

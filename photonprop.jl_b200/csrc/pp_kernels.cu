@@ -19,6 +19,7 @@
 
 #include "pp_device.cuh"
 #include "pp_internal.h"
+#include "pp_special.cuh"
 
 namespace ppd {
 
@@ -649,6 +650,12 @@ __global__ void normalize_kernel(const pp_pair* __restrict__ pairs, int64_t n_pa
 __global__ void eval_kernel(int op, const double* __restrict__ in, double* __restrict__ out, int64_t n,
                             const DevTables* __restrict__ tables) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (op == 13 || op == 14) {  // a warp's lanes hold the tables: all take part
+    const ppsf::WarpTables W = ppsf::warp_tables();
+    const double v = in[min(i, n - 1)], r = op == 13 ? ppsf::exp_tab(v, W) : ppsf::log_tab(v, W);
+    if (i < n) out[i] = r;
+    return;
+  }
   if (i >= n) return;
   const DevTables& T = *tables;
   switch (op) {
@@ -701,6 +708,8 @@ __global__ void eval_kernel(int op, const double* __restrict__ in, double* __res
     case 7: out[i] = (double)group_index(T, 1.f / (float)in[i]); break;
     case 8: out[i] = (double)scattering_length(T, (float)in[i]); break;
     case 9: out[i] = (double)interp_sorted((float)in[i], T.abs_wl, T.abs_len, T.n_abs); break;
+    case 15: ppsf::psi_both(in[i], out[2 * i], out[2 * i + 1]); break;
+    case 16: out[i] = ppsf::reciprocal_1_2(in[i]); break;
     case 11: out[i] = (double)cascade_cos_theta(T, 1.f / (float)in[2 * i + 1], (float)in[2 * i]); break;
     case 10:
       out[i] = T.n_pmt > 0 ? (double)interp_sorted((float)in[i], T.pmt_wl, T.pmt_acc, T.n_pmt) : 1.0;

@@ -1030,17 +1030,6 @@ __device__ __forceinline__ double inv_digamma(double y, Psi& P, bool active) {
   }
 }
 
-// 1 / s for 1 <= s <= 2, within 1 ulp: the FP32 reciprocal of its leading
-// bits (2^-20) and one step of Newton's iteration, third order.
-__device__ __forceinline__ double reciprocal_1_2(double s) {
-  const float f = __uint_as_float(__funnelshift_l(__double2loint(s), __double2hiint(s), 3) + 0x40000000u);
-  float g;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(g) : "f"(f));
-  const double r = __hiloint2double((int)((__float_as_uint(g) >> 3) + 0x38000000u), 0);
-  const double e = fma(-s, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-
 __global__ void __launch_bounds__(kMixWarps * 32, 1) gamma_fit_kernel(const double* __restrict__ hist, int64_t n, int bins,
                                                                      float t0, float bw,
                                                                      const float* __restrict__ tshift,
@@ -1160,7 +1149,7 @@ __global__ void __launch_bounds__(kMixWarps * 32, 1) gamma_fit_kernel(const doub
           }
 #pragma unroll
           for (int q = 0; q < Q; ++q) {
-            const double v = reciprocal_1_2(1.0 + e[q]);
+            const double v = ppsf::reciprocal_1_2(1.0 + e[q]);
             const double f = d[q] > 0 ? v : e[q] * v;  // component 1's share
             // 1 - f, which is 0 once component 2 falls below the rounding of 1:
             // its parameters then stay as they are

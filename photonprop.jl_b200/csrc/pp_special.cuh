@@ -2,8 +2,8 @@
 // asymptotic series
 //   psi(x)  = ln x - 1/(2x) - sum_k B_2k / (2k x^2k)
 //   psi'(x) = 1/x + 1/(2x^2) + sum_k B_2k / x^(2k+1)
-// (Bernoulli numbers to B_10, B_8 for the second): within 1e-11 and 3e-10 at
-// x = 6, less above.
+// (Bernoulli numbers to B_10, B_8 for the second): within 1e-11 and 3e-10
+// (absolute, at x = 6; largest seen 8.8e-12 and 1.9e-10), less above.
 #pragma once
 
 namespace ppsf {
@@ -30,7 +30,9 @@ __device__ __forceinline__ void psi_both(double x, double& psi, double& psi1) {
 // 144 and 16 (1990) 378): the argument is reduced to 1/32 of an octave, the
 // remainder's Taylor series needs few terms, and a warp's 32 lanes hold the
 // table, one entry each, which a lookup takes by shuffle (all lanes take part).
-// Against the FP64 values: exp within 1 ulp, log within 2e-16 + 1 ulp.
+// exp within 1.6 ulp (the table's entry 1, the last rounding 0.5; largest
+// seen 1.09), log within 2e-16 (the table's entry) + 1.5 ulp (ln 2 times the
+// exponent, two roundings; largest seen 1.3e-16 in [0.5, 2], 1.27 ulp beyond).
 struct WarpTables {
   double exp2_at;         // 2^(lane / 32)
   double inv_at, log_at;  // 1 / c, rounded to FP32, and ln c, for c at the middle of [1 + lane/32, 1 + (lane + 1)/32)
@@ -104,6 +106,17 @@ __device__ __forceinline__ double log_tab(double y, const WarpTables& T) {
   q = fma(r, q, T.l3);
   q = fma(r, q, -0.5);
   return fma(k, T.ln2, __shfl_sync(0xffffffffu, T.log_at, at)) + fma(r * r, q, r);
+}
+
+// 1 / s for 1 <= s <= 2, within 1 ulp (largest seen 0.502): the FP32 reciprocal of its leading
+// bits (2^-20) and one step of Newton's iteration, third order.
+__device__ __forceinline__ double reciprocal_1_2(double s) {
+  const float f = __uint_as_float(__funnelshift_l(__double2loint(s), __double2hiint(s), 3) + 0x40000000u);
+  float g;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(g) : "f"(f));
+  const double r = __hiloint2double((int)((__float_as_uint(g) >> 3) + 0x38000000u), 0);
+  const double e = fma(-s, r, 1.0);
+  return fma(r, fma(e, e, e), r);
 }
 
 }  // namespace ppsf

@@ -248,7 +248,7 @@ class Propagator:
         return n.value
 
     def device_eval(self, op: int, inputs) -> np.ndarray:
-        out_w = {0: 4, 3: 3, 4: 3, 12: 5}.get(op, 1)
+        out_w = {0: 4, 3: 3, 4: 3, 12: 5, 15: 2}.get(op, 1)
         x = np.ascontiguousarray(inputs, dtype=np.float64)
         n = x.shape[0] if x.ndim > 0 else 1
         out = np.zeros((n, out_w))
