@@ -516,6 +516,10 @@ PP_API pp_status pp_mlp_train_step(pp_mlp* m, const float* d_xn, const float* d_
 /* One 128 x 128 x 128 BF16 GEMM (c = a b^T, row-major) through the tcgen05
  * path: a check of the tensor-core descriptors. */
 PP_API pp_status pp_mlp_gemm_selftest(int device, const uint16_t* a_bf16, const uint16_t* b_bf16, float* c);
+/* The same for each operand layout that training uses: 0 c = a b^T (a layer
+ * forward), 1 c = a b (dh = dz W), 2 c = a^T b (dW = dz^T h). */
+PP_API pp_status pp_mlp_gemm_selftest_layout(int device, int32_t layout, const uint16_t* a_bf16,
+                                             const uint16_t* b_bf16, float* c);
 
 /* Fits w G(a1, theta) + (1 - w) G(a2, theta) to each of n histograms
  * (device, FP64 [n][bins], bin b centred at t0 + (b + 1/2) bin_width) as a

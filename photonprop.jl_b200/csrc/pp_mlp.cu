@@ -56,16 +56,9 @@ __device__ __forceinline__ void gelu_both(float z, float& h, float& g) {
 // error below 2^-10, under the BF16 rounding that follows it), in four FP32
 // operations: u = z (k + k c z^2), 2 GELU = z (1 + t).  The factor 1/2 is
 // folded into the next layer's weights (exact: a power of two commutes with
-// the BF16 rounding of both the weights and the activations).
-__device__ __forceinline__ float gelu2_fast(float z) {
-  const float u = z * fmaf(0.7978845608028654f * 0.044715f, z * z, 0.7978845608028654f);
-  float t;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(u));
-  return fmaf(z, t, z);
-}
-// The same arithmetic on two activations at once with sm_100's packed FP32
-// instructions (round to nearest, so bit for bit the scalar result): half the
-// FP32 issue slots of the epilogue.
+// the BF16 rounding of both the weights and the activations).  Two activations
+// at once with sm_100's packed FP32 instructions: half the FP32 issue slots of
+// the epilogue.
 __device__ __forceinline__ float2 gelu2_fast2(float2 z) {
   constexpr float k0 = 0.7978845608028654f, k1 = 0.7978845608028654f * 0.044715f;
   const float2 k = __ffma2_rn(__fmul2_rn(z, z), make_float2(k1, k1), make_float2(k0, k0));
@@ -89,12 +82,6 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 // Instruction descriptor: D = F32, A = B = BF16, both K-major, N = 128, M = 128.
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 
-__device__ __forceinline__ void mma_128x128x16(uint32_t tmem, uint64_t a, uint64_t b, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem),
-      "l"(a), "l"(b), "r"(kIdesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
-}
 __device__ __forceinline__ void mma_commit(uint32_t mbar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
                : "memory");
@@ -150,16 +137,18 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// Tensor-memory allocation of 128 columns by warp 0; the address lands in *slot.
+// Tensor-memory allocation of COLS columns by warp 0; the address lands in *slot.
+template <int COLS>
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot) {
   if ((threadIdx.x >> 5) == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;" ::"r"(smem_u32(slot)));
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "n"(COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
 }
+template <int COLS>
 __device__ __forceinline__ void tmem_free(uint32_t taddr) {
   if ((threadIdx.x >> 5) == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(taddr));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "n"(COLS));
 }
 
 // Writes 8 consecutive columns [k8*8, k8*8+8) of `row` (FP32 values, rounded
@@ -169,28 +158,6 @@ __device__ __forceinline__ void store8(__nv_bfloat16* tile, int row, int k8, con
 #pragma unroll
   for (int i = 0; i < 4; ++i) p[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
   *reinterpret_cast<int4*>(tile + tc_offset(row, k8 * 8)) = *reinterpret_cast<int4*>(p);
-}
-
-// D[128 x 128] (TMEM) = A (tile a, rows x K) * B^T (tile b, N rows x K), issued
-// by thread 0 after every thread's shared-memory writes are fenced and synced.
-// Returns false if the wait expired.
-__device__ __forceinline__ bool tile_gemm(const __nv_bfloat16* a, const __nv_bfloat16* b, uint32_t tmem,
-                                          uint32_t mbar, uint32_t& parity) {
-  fence_async_smem();
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  if (threadIdx.x == 0) {
-    const uint32_t sa = smem_u32(a), sb = smem_u32(b);
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      mma_128x128x16(tmem, smem_desc(sa + k * 256, 128, 2048), smem_desc(sb + k * 256, 128, 2048), k > 0);
-    mma_commit(mbar);
-  }
-  const bool ok = mbar_wait(mbar, parity);
-  parity ^= 1u;
-  tc_fence_after();
-  return ok;
 }
 
 // element offset of (row, k) in a K-major canonical tile of 16 columns
@@ -217,8 +184,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
-
-__device__ __forceinline__ uint32_t lane_taddr(uint32_t tmem) { return tmem + ((threadIdx.x & ~31u) << 16); }
 
 // ---------------------------------------------------------------------------
 // Device parameter block.
@@ -343,10 +308,7 @@ __global__ void __launch_bounds__(INFER_THREADS, 1) infer_kernel(DevParams P, co
   if (t < OUT) b4[t] = P.p[OFF_B4 + t];
   if (t < 18) nrm[t] = P.norm[t];
   if (t < IN) nrm[18 + t] = 1.f / P.norm[4 + t];  // feature scales as reciprocals: no division per row
-  if ((t >> 5) == 0) {  // all 512 columns: 128 per group
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tslot)));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
+  tmem_alloc<512>(tslot);  // 128 columns per group
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -483,7 +445,7 @@ __global__ void __launch_bounds__(INFER_THREADS, 1) infer_kernel(DevParams P, co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if ((t >> 5) == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base));
+  tmem_free<512>(tmem_base);
 }
 
 // ---------------------------------------------------------------------------
@@ -549,6 +511,14 @@ __device__ __forceinline__ void bulk_add_row(float* dst, const void* src) {
                : "memory");
 }
 
+// The k-th 16 of K of an operand tile: read K-major, or as MN-major (neighbouring
+// 8-column groups 128 B apart, 8-row groups, K then, 2048 B).
+__device__ __forceinline__ uint64_t kmaj(const __nv_bfloat16* tile, int k) {
+  return smem_desc(smem_u32(tile) + k * 256, 128, 2048);
+}
+__device__ __forceinline__ uint64_t mn(const __nv_bfloat16* tile, int k) {
+  return smem_desc(smem_u32(tile) + k * 4096, 2048, 128);
+}
 // A and B both MN-major (bits 15 and 16), or B alone.
 constexpr uint32_t kIdescMnMn = kIdesc | (1u << 15) | (1u << 16), kIdescKMn = kIdesc | (1u << 16);
 
@@ -623,10 +593,7 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1) train_kernel(DevParams P, co
   for (int j = 0; j < IN; ++j) x[j] = valid ? bf16r(xn[row * IN + j]) : 0.f;
   if (c0 == 0) *reinterpret_cast<float4*>(xs + r * IN) = make_float4(x[0], x[1], x[2], x[3]);
   if (t == 0) mbar_init(smem_u32(mbar));
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tslot)));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
+  tmem_alloc<512>(tslot);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -658,9 +625,6 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1) train_kernel(DevParams P, co
 #pragma unroll
     for (int q = 0; q < 4; ++q) store8(tile, r, c0 / 8 + q, v + q * 8);
   };
-  // operand tile as MN-major: neighbouring 8-column groups 128 B apart, 8-row groups (K) 2048 B
-  auto mn = [&](const __nv_bfloat16* tile, int k) { return smem_desc(smem_u32(tile) + k * 4096, 2048, 128); };
-  auto kmaj = [&](const __nv_bfloat16* tile, int k) { return smem_desc(smem_u32(tile) + k * 256, 128, 2048); };
 
   // ---- forward
   {
@@ -867,7 +831,7 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1) train_kernel(DevParams P, co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tm));
+  tmem_free<512>(tm);
 }
 
 // The BF16 copies of the master parameters that the tensor cores read.
@@ -926,9 +890,10 @@ __global__ void __launch_bounds__(256) prepare_kernel(const float* __restrict__ 
   if (i < N_PARAMS) write_copies(C, i, p[i]);
 }
 
-// One 128 x 128 x 128 GEMM through the tensor-core path (descriptor self-test):
-// c[i][j] = sum_k a[i][k] b[j][k], a and b BF16 row-major, c FP32.
-__global__ void __launch_bounds__(THREADS, 1) gemm_test_kernel(const __nv_bfloat16* __restrict__ a,
+// One 128 x 128 x 128 GEMM with the descriptors that training uses, a and b
+// BF16 row-major, c FP32: layout 0 a b^T (a layer), 1 a b (dh = dz W), 2 a^T b
+// (dW = dz^T h).
+__global__ void __launch_bounds__(THREADS, 1) gemm_test_kernel(int layout, const __nv_bfloat16* __restrict__ a,
                                                               const __nv_bfloat16* __restrict__ b,
                                                               float* __restrict__ c, int* error) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -942,17 +907,26 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_test_kernel(const __nv_bfloat
     tb[tc_offset(t, k)] = b[t * H + k];
   }
   if (t == 0) mbar_init(smem_u32(mbar));
-  tmem_alloc(tslot);
+  tmem_alloc<128>(tslot);
+  fence_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tslot;
-  uint32_t parity = 0;
-  const bool ok = tile_gemm(ta, tb, tmem, smem_u32(mbar), parity);
+  if (t == 0) {
+    for (int k = 0; k < 8; ++k) {
+      if (layout == 0) mma_idesc(tmem, kmaj(ta, k), kmaj(tb, k), kIdesc, k > 0);
+      if (layout == 1) mma_idesc(tmem, kmaj(ta, k), mn(tb, k), kIdescKMn, k > 0);
+      if (layout == 2) mma_idesc(tmem, mn(ta, k), mn(tb, k), kIdescMnMn, k > 0);
+    }
+    mma_commit(smem_u32(mbar));
+  }
+  const bool ok = __syncthreads_and(mbar_wait(smem_u32(mbar), 0));
+  tc_fence_after();
   if (ok) {
     for (int q = 0; q < 4; ++q) {
       float v[32];
-      tmem_ld32(lane_taddr(tmem) + q * 32, v);
+      tmem_ld32(tmem + ((uint32_t)(t & ~31) << 16) + q * 32, v);
       for (int i = 0; i < 32; ++i) c[t * H + q * 32 + i] = v[i];
     }
   } else if (t == 0) {
@@ -961,7 +935,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_test_kernel(const __nv_bfloat
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  tmem_free(tmem);
+  tmem_free<128>(tmem);
 }
 
 // ---------------------------------------------------------------------------
@@ -1494,7 +1468,12 @@ pp_status pp_mlp_train_step(pp_mlp* m, const float* d_xn, const float* d_yt, con
 }
 
 pp_status pp_mlp_gemm_selftest(int device, const uint16_t* a_bf16, const uint16_t* b_bf16, float* c) {
-  if (!a_bf16 || !b_bf16 || !c) return PP_ERR_ARG;
+  return pp_mlp_gemm_selftest_layout(device, 0, a_bf16, b_bf16, c);
+}
+
+pp_status pp_mlp_gemm_selftest_layout(int device, int32_t layout, const uint16_t* a_bf16, const uint16_t* b_bf16,
+                                      float* c) {
+  if (!a_bf16 || !b_bf16 || !c || layout < 0 || layout > 2) return PP_ERR_ARG;
   Guard g(device);
   void *da = nullptr, *db = nullptr, *dc = nullptr, *de = nullptr;
   cudaError_t e;
@@ -1510,7 +1489,7 @@ pp_status pp_mlp_gemm_selftest(int device, const uint16_t* a_bf16, const uint16_
   cudaMemcpy(da, a_bf16, 128 * 128 * 2, cudaMemcpyHostToDevice);
   cudaMemcpy(db, b_bf16, 128 * 128 * 2, cudaMemcpyHostToDevice);
   cudaMemset(de, 0, 16);
-  mlp::gemm_test_kernel<<<1, mlp::THREADS, mlp::kTestSmem>>>(static_cast<const __nv_bfloat16*>(da),
+  mlp::gemm_test_kernel<<<1, mlp::THREADS, mlp::kTestSmem>>>(layout, static_cast<const __nv_bfloat16*>(da),
                                                              static_cast<const __nv_bfloat16*>(db),
                                                              static_cast<float*>(dc), static_cast<int*>(de));
   pp::count_launches(1);

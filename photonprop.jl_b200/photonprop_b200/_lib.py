@@ -163,6 +163,7 @@ _SIGS = [
     ("pp_mlp_train_step", ctypes.c_int, [_VP, _VP, _VP, _VP, _I64, ctypes.c_float, ctypes.POINTER(ctypes.c_float),
                                          _VP]),
     ("pp_mlp_gemm_selftest", ctypes.c_int, [ctypes.c_int, _VP, _VP, _VP]),
+    ("pp_mlp_gemm_selftest_layout", ctypes.c_int, [ctypes.c_int, _I32, _VP, _VP, _VP]),
     ("pp_gamma_mixture_fit", ctypes.c_int, [_VP, _I64, _I32, ctypes.c_float, ctypes.c_float, _VP, _VP, _I32, _VP]),
     ("pp_autotune", ctypes.c_int, [_VP, _VP, _I64, ctypes.POINTER(RunOpts), ctypes.c_char_p,
                                    ctypes.POINTER(RunOpts), ctypes.POINTER(_D)]),

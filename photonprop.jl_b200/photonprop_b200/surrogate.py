@@ -91,13 +91,14 @@ class MLP:
         return float(loss.value), g
 
 
-def gemm_selftest(a_bf16_u16, b_bf16_u16, device=0):
-    """c = a b^T through the tcgen05 path (a, b uint16 BF16 bit patterns [128,128])."""
+def gemm_selftest(a_bf16_u16, b_bf16_u16, device=0, layout=0):
+    """c = a b^T through the tcgen05 path (a, b uint16 BF16 bit patterns [128,128]); layout 1: a b, 2: a^T b, with
+    the descriptors of training's backward pass."""
     L = _lib.load()
     a = np.ascontiguousarray(a_bf16_u16, dtype=np.uint16)
     b = np.ascontiguousarray(b_bf16_u16, dtype=np.uint16)
     c = np.zeros((128, 128), dtype=np.float32)
-    _lib.check(L.pp_mlp_gemm_selftest(device, a.ctypes.data, b.ctypes.data, c.ctypes.data))
+    _lib.check(L.pp_mlp_gemm_selftest_layout(device, layout, a.ctypes.data, b.ctypes.data, c.ctypes.data))
     return c
 
 
