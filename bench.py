@@ -818,8 +818,8 @@ def run_reference(args):
 def plain_by_pair_size(prop, ro, b, d_batch, d_pair_views, h_pairs, d_hits, cap, d_cnt, d_st1, d_hi1, d_stats,
                        d_hist, s, flush):
     """Where the one-pair-per-launch path loses against the batched kernel:
-    per-pair device time of the plain path (its memsets, counter reset,
-    kernel and finalisation, launched back to back as in the plain pass) and
+    per-pair device time of the plain path (its set-up and its kernel,
+    launched back to back as in the plain pass) and
     the batched kernel on each photon-count decade of the same batch alone,
     photons/s per decade, plus the plain path's fixed cost per pair (the
     median time of the pairs below 2e4 photons)."""
@@ -834,7 +834,7 @@ def plain_by_pair_size(prop, ro, b, d_batch, d_pair_views, h_pairs, d_hits, cap,
         ev[i][1].record(s)
     s.synchronize()
     t = np.array([a.elapsed_time(e) / 1e3 for a, e in ev])
-    out = {"what": "plain: per-pair device time (memsets, reset, kernel, finalisation) summed per decade; batched: "
+    out = {"what": "plain: per-pair device time (set-up, kernel) summed per decade; batched: "
                    "the decade's pairs as one batched launch",
            "plain_fixed_cost_us_per_pair": float(np.median(t[n < 20000]) * 1e6) if np.any(n < 20000) else None,
            "decades": []}
@@ -1001,9 +1001,11 @@ def run_ours(args):
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         with torch.cuda.stream(s):
             flush.fill_(1)
+        plain_launches = pp.launch_count()
         e0.record(s)
         plain_pass()
         e1.record(s)
+        plain_launches = pp.launch_count() - plain_launches
         s.synchronize()
         t_pk = e0.elapsed_time(e1) / 1e3
         hits_np = np.zeros(cap, dtype=pp.HIT_DTYPE)
@@ -1015,7 +1017,7 @@ def run_ours(args):
         ph = photons_local[0]
         plain = {"kernel_photons_per_s": reduce(ph, SUM) / reduce(t_pk, MAX),
                  "host_api_photons_per_s": reduce(ph, SUM) / reduce(t_ph, MAX),
-                 "launches_per_pass": 3 * n_pairs}
+                 "launches_per_pass": plain_launches}
         plain["batched_over_plain_kernel"] = value / plain["kernel_photons_per_s"]
         plain["batched_over_plain_host_api"] = value / plain["host_api_photons_per_s"]
         plain["by_pair_size"] = plain_by_pair_size(prop, ro, b, d_pairs[W], d_pair_views, h_pairs, d_hits, cap,
@@ -1121,7 +1123,7 @@ def run_ours(args):
                      "peak_source": "measured live: ex2.approx dependent chains over every SM (pp_measure_peaks)",
                      "counts": "achieved = MUFU operations of the steps made, in the reference's arithmetic (7 per "
                                "photon step, 10 per isotropic / 14 per cone photon start), per second; 'issued' = "
-                               "this kernel's own count (7 MUFU and 46 FP32 per step, ncu opcode counts); "
+                               "this kernel's own count (6 MUFU and 46 FP32 per step, ncu opcode counts); "
                                "'algorithmic' = with the steps that the reach test spares (one per photon that ends "
                                "out of reach), which no kernel makes",
                      "issued": {"mufu_achieved": mufu_i / t_local / 1e9,
@@ -1141,7 +1143,7 @@ def run_ours(args):
                          "what": "bare physical step on every SM (Philox block, ray-sphere, move, turn; no emission, "
                                  "refill, hits or loop bookkeeping), pp_measure_step_rate",
                          "mufu_frac_ceiling": roofline.MUFU_PER_STEP_ALG * sol_steps / peaks["mufu_ops"],
-                         "mufu_frac_ceiling_issued": roofline.MUFU_PER_STEP * sol_steps / peaks["mufu_ops"],
+                         "mufu_frac_ceiling_issued": roofline.MUFU_PER_BARE_STEP * sol_steps / peaks["mufu_ops"],
                          "batched_steps_frac": steps_total / t_local / sol_steps,
                          "frac_of_ceiling": f_mufu / (roofline.MUFU_PER_STEP_ALG * sol_steps / peaks["mufu_ops"])},
                      "hbm": {"achieved_gbs": alg_bytes / t_local / 1e9, "peak_gbs": measured_hbm_gbs(),

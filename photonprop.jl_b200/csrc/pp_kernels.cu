@@ -51,18 +51,21 @@ namespace ppd {
 // fast as the ring at any share (24.1 against 46.4 ms at 80 %), and its kernel
 // without the other loop (THIN) 2 % faster on 2e7 photons.
 //
-// Bound by instruction issue (77 % of the issue slots, ALU half-rate pipe
-// 50 %); what counts is instructions per photon.  512 mixed pairs (1.1e8
-// photons): 3.00e9 -> 2.36e9 warp instructions, 3.47 -> 2.85 ms, by testing
+// Bound by instruction issue (78 % of the issue slots, ALU half-rate pipe
+// 48 %); what counts is instructions per photon.  512 mixed pairs (2.52e8
+// photons): 6.30e9 -> 4.94e9 warp instructions, 6.99 -> 5.57 ms, by testing
 // the reach where a photon stops (in_reach), one emission pass per pair with
 // its record by broadcast, and separate loops for the full warp and for the
-// last photons; 4096 mixed pairs (5.75e9 photons): 171 -> 139 ms.  Compat mode
-// (100 distances, 2e9 photons): 139.4 -> 90.1 ms, 124 warp instructions per
-// step with the emission's tenth and the hits; the last step leaves out the
-// move and turn that nothing follows, steps are counted by what hits leave
-// out, a batch of hits adds its sums over the warp.  Measured and not kept:
-// the first one or two steps of physical mode inside the emission
-// pass (fewer loop iterations, but 180 bytes spilled at 64 registers: 3.26 ms).
+// last photons; 4096 mixed pairs (5.75e9 photons): 171 -> 138 ms.  Cascade
+// pairs: 25.3 warp instructions per photon against 19.6 of the mixed batch
+// (3.68 steps against 3.37, a longer emission; its table reads hit L1 and do
+// not stall), issue 75 %.  Compat mode (100 distances, 2e9 photons): 139.4 ->
+// 90.1 ms, 124 warp instructions per step with the emission's tenth and the
+// hits; the last step leaves out the move and turn that nothing follows, steps
+// are counted by what hits leave out, a batch of hits adds its sums over the
+// warp.  Measured and not kept: the first one or two steps of physical mode
+// inside the emission pass (fewer loop iterations, but 180 bytes spilled at 64
+// registers: 14 % slower).
 constexpr int kStage = 64;  // >= 2 * 32 - 1 staged emissions per warp (power of two)
 
 constexpr unsigned kThinLive = 16, kRefill = 8;

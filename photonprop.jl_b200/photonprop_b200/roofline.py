@@ -6,12 +6,15 @@ per photon step   7 MUFU  the reference's arithmetic (src/photon_prop_cuda.jl:
                           azimuth, sqrt(1 - o_z^2) and rsqrt in the rotation (its
                           two divisions by sin(theta) share one rcp), plus the
                           square root of the ray-sphere discriminant when the
-                          line meets the sphere; the roofline counts 7.  This
-                          kernel issues 7 as well (lg2, sqrt of the
-                          discriminant, rcp, sqrt, sin, cos and the turn's
-                          rsqrt in physical mode, rcp in the compat-mode
-                          rotation), which ncu's opcode counts of the
-                          bare-step kernel confirm.
+                          line meets the sphere; the roofline counts 7.  The
+                          bare step issues 7 (lg2, sqrt of the discriminant,
+                          rcp, sqrt, sin, cos and the turn's rsqrt in physical
+                          mode, rcp in the compat-mode rotation; ncu opcode
+                          counts).  The batched kernel issues 6: it takes the
+                          discriminant's root under a branch, which few warps
+                          enter (512 mixed pairs, 2.524e8 photons: 2.549e8 MUFU
+                          warp instructions = 7.89e6 emission passes x 12 and
+                          2.70e7 warp steps x 6 within 1 %).
                  ~45 FP32 in the reference's form; this kernel issues 46
                           (ncu: 24 FFMA, 17 FMUL, 5 FADD per step; the
                           physical-mode turn in the meridian frame, without
@@ -25,7 +28,8 @@ A photon that hits the sphere also re-draws its emission block (rare).
 
 MUFU_PER_STEP_ALG = 7
 FP32_PER_STEP_ALG = 45
-MUFU_PER_STEP = 7
+MUFU_PER_STEP = 6
+MUFU_PER_BARE_STEP = 7
 FP32_PER_STEP = 46
 PHILOX_PER_STEP = 0.5  # Philox4x32-10 block equivalents (by 32x32-bit products)
 MUFU_PER_PHOTON = {0: 10, 1: 14}   # by emitter type
@@ -53,6 +57,6 @@ def op_counts(steps, photons_iso, photons_cone, algorithmic=False):
 # stays in the 126 MB L2 during the launch and reaches DRAM afterwards.
 NCU_DRAM_BYTES_PER_LAUNCH = 0.5 * ((2.08 + 22.35) + (2.57 + 30.91)) * 1e6
 # Issue and pipes on one launch of 512 mixed pairs (<= 1e6 photons each).
-NCU_ISSUE_ACTIVE = 0.777
-NCU_PIPES = {"alu": 0.478, "fma": 0.421, "xu": 0.406}  # pipe utilisation, same capture
-NCU_LANES_ACTIVE = 30.59  # threads per executed warp instruction, same capture
+NCU_ISSUE_ACTIVE = 0.778
+NCU_PIPES = {"alu": 0.478, "fma": 0.418, "xu": 0.407}  # pipe utilisation, same capture
+NCU_LANES_ACTIVE = 30.58  # threads per executed warp instruction, same capture
